@@ -1,0 +1,49 @@
+"""The forms staged in shared memory by TMA that the default tuning runs: the VI and FDK
+backprojectors (csrc/vi_tma.cu), against the forms that read global memory."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def tomo():
+    import tomogpi_b200 as t
+
+    return t
+
+
+def _cfg(t, nx, ny, nz, nu, nv, views, pitch, mag=2.0, fod=None):
+    fod = 2.0 * max(nx, ny) if fod is None else fod
+    return t.ConfigCT(fod=fod, fdd=mag * fod, projection_nb=views, u_detector_size=pitch * nu, v_detector_size=pitch * nv,
+                      u_detector_pixel_nb=nu, v_detector_pixel_nb=nv, x_volume_size=float(nx), y_volume_size=float(ny),
+                      z_volume_size=float(nz), x_volume_pixel_nb=nx, y_volume_pixel_nb=ny, z_volume_pixel_nb=nz)
+
+
+# 4, 8 and 16 slices per thread (64^3, 128^3, 160^3), partial tiles and chunks, detector
+# widths 0..3 modulo 4, a steep cone (windows beyond the box), a detector smaller than the
+# volume's shadow
+VI = [(64, 64, 64, 64, 64, 9, 2.0), (128, 128, 128, 130, 126, 5, 2.0), (160, 157, 161, 163, 141, 5, 2.0),
+      (33, 41, 18, 47, 29, 7, 1.7), (96, 96, 200, 129, 240, 6, 3.0, 2.5, 80.0), (130, 130, 90, 61, 40, 6, 2.0)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("spec", VI, ids=lambda s: "x".join(map(str, s)))
+def test_staged_backprojection_equals_padded(tomo, spec, dtype):
+    """VI and its UM variant: bit-identical to the padded copy's kernel (32 slices per thread).
+    FDK: the weights' reciprocal square root is within 2 ulp, so 1e-6 of the padded kernel."""
+    cfg = _cfg(tomo, *spec)
+    sino = torch.from_numpy(np.random.default_rng(5).random(cfg.sinogram_shape, dtype=np.float32)).cuda().to(dtype)
+    with tomo.Context(cfg) as ctx:
+        got = {k: ctx.backproject(k, sino, dtype=torch.float32) for k in ("VI", "VI_UM", "FDK")}
+        ctx.set_tuning(vi_zc=2)
+        for k, v in got.items():
+            ref = ctx.backproject(k, sino, dtype=torch.float32)
+            assert float(ref.abs().max()) > 0
+            if k == "FDK":
+                assert float(torch.linalg.vector_norm((v - ref).double()) / torch.linalg.vector_norm(ref.double())) <= 1e-6
+            else:
+                assert torch.equal(v, ref), k
+        torch.cuda.synchronize()
+        assert ctx.errors() == 0

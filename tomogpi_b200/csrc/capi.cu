@@ -44,6 +44,7 @@ struct tomo_context {
     unsigned long long* d_count = nullptr;
     void* vpad[3] = {nullptr, nullptr, nullptr};  // padded volume per storage dtype
     void* spad[3] = {nullptr, nullptr, nullptr};  // padded sinogram per storage dtype
+    float* rows = nullptr;                         // FP32 sinogram rows for the TMA-staged VI
     float* adj_scratch = nullptr;                  // FP32 volume for adjoints into 16-bit outputs
     float* h_vol = nullptr;                        // device buffers of the host-buffer forms
     float* h_sino = nullptr;
@@ -60,6 +61,7 @@ struct tomo_context {
     size_t nvox() const { return (size_t)hg.nx * hg.ny * hg.nz; }
     size_t nsino() const { return (size_t)hg.nu * hg.nv * hg.np; }
     size_t nvox_pad() const { return (size_t)(hg.nx + 2) * (hg.ny + 2) * (hg.nz + 2); }
+    size_t nsino_rows() const { return (size_t)vi_rows_pitch(hg.nu) * hg.nv * hg.np; }
     size_t nsino_pad() const { return (size_t)(hg.nu + 2) * (hg.nv + 2) * hg.np; }
 };
 
@@ -142,6 +144,11 @@ OutView<void> plain_view(void* p, const HostGeom& h) {
     return OutView<void>{p, 0, (long)h.nu, (long)h.nu * h.nv};
 }
 
+OutView<void> rows_view(void* p, const HostGeom& h) {
+    const long W = vi_rows_pitch(h.nu);
+    return OutView<void>{p, 0, W, W * h.nv};
+}
+
 OutView<void> padded_view(void* p, const HostGeom& h) {
     const long W = h.nu + 2;
     return OutView<void>{p, W + 1, W, W * (h.nv + 2)};
@@ -151,6 +158,13 @@ OutView<void> padded_view(void* p, const HostGeom& h) {
 // that layout is off or the view count exceeds the layer limit.
 bool vi_texture(const tomo_context* ctx) {
     return ctx->tuning.vi_layout == 1 && ctx->hg.np <= rs_tex_max_layers();
+}
+
+// The VI and FDK backprojectors stage detector windows by TMA in the default form (padded, 16
+// slices per thread) as in the "tma" form; other chunkings read the padded copy.
+bool vi_staged(const tomo_context* ctx) {
+    return (ctx->tuning.vi_layout == 2 || (ctx->tuning.vi_layout == 0 && ctx->tuning.vi_zc == 1)) &&
+           vi_tma_supported(nullptr, 4);
 }
 
 // The RS layout actually used: the texture layouts need an array layer per z slice (plus
@@ -292,6 +306,7 @@ tomo_status tomo_context_destroy(tomo_context* ctx) {
         cudaFree(ctx->vpad[i]);
         cudaFree(ctx->spad[i]);
     }
+    cudaFree(ctx->rows);
     cudaFree(ctx->adj_scratch);
     rs_tex_destroy(&ctx->tex);
     rs_tex_destroy(&ctx->vtex);
@@ -390,11 +405,27 @@ tomo_status tomo_backproject(tomo_context* ctx, tomo_backprojector kind, const v
                                                volume_dtype, 1.0f, st, ctx->tuning.vi_zc),
                             "vi_back_tex_kernel");
     }
-    if ((kind == TOMO_BACK_VI || kind == TOMO_BACK_VI_UM) && ctx->tuning.vi_layout == 2 &&
-        sinogram_dtype == TOMO_F32 && vi_tma_supported(g, sinogram))  // the caller's sinogram, no padded copy
-        return check_launch(launch_vi_back_tma(kind == TOMO_BACK_VI_UM ? 1 : 0, g, (const float*)sinogram, volume,
-                                               volume_dtype, 1.0f, ctx->d_err, st, ctx->test_stall),
-                            "vi_back_tma_kernel");
+    if ((kind == TOMO_BACK_VI || kind == TOMO_BACK_VI_UM || kind == TOMO_BACK_FDK) && vi_staged(ctx)) {
+        // the caller's FP32 rows where a tensor map can describe them, else a copy (one without
+        // memory for the copy takes the padded form, whose 16-bit copy is half the size)
+        const float* rows = (const float*)sinogram;
+        long pitch = g.nu;
+        if (sinogram_dtype != TOMO_F32 || !vi_tma_supported(sinogram, g.nu)) {
+            pitch = vi_rows_pitch(g.nu);
+            if (!ctx->rows && cudaMalloc((void**)&ctx->rows, (size_t)pitch * g.nv * g.np * sizeof(float)) != cudaSuccess) {
+                cudaGetLastError();
+                ctx->rows = nullptr;
+            }
+            rows = ctx->rows;
+            if (rows && (s = check_launch(launch_sino_rows(sinogram, sinogram_dtype, ctx->rows, g.nu, g.nv, g.np, (int)pitch, st),
+                                          "sinogram rows")) != TOMO_OK)
+                return s;
+        }
+        if (rows)
+            return check_launch(launch_vi_back_tma(kind == TOMO_BACK_FDK ? 2 : kind == TOMO_BACK_VI_UM ? 1 : 0, g, rows, pitch,
+                                                   volume, volume_dtype, 1.0f, ctx->d_err, st, ctx->test_stall),
+                                "vi_back_tma_kernel");
+    }
     if (kind == TOMO_BACK_FDK) {
         s = ensure(&ctx->spad[sinogram_dtype], ctx->nsino_pad() * dtype_size(sinogram_dtype), true);
         if (s != TOMO_OK) return s;
@@ -564,7 +595,7 @@ tomo_status tomo_solver_create(tomo_context* ctx, const tomo_gradient_params* pr
         if (zero && cudaMemset(*p, 0, bytes) != cudaSuccess) return false;
         return true;
     };
-    bool ok = alloc(&sv->vpad, rs_input_elems(sv->rs_layout, ctx->hg.nx, ctx->hg.ny, ctx->hg.nz) * es, true) && alloc(&sv->spad, ctx->nsino_pad() * sizeof(float), true) &&
+    bool ok = alloc(&sv->vpad, rs_input_elems(sv->rs_layout, ctx->hg.nx, ctx->hg.ny, ctx->hg.nz) * es, true) && alloc(&sv->spad, std::max(ctx->nsino_pad(), ctx->nsino_rows()) * sizeof(float), true) &&
               alloc((void**)&sv->dJ, ctx->nvox() * sizeof(float), false) &&
               alloc((void**)&sv->grad, ctx->nvox() * sizeof(float), false) &&
               alloc((void**)&sv->nrm, 8 * sizeof(double), true) && alloc((void**)&sv->state, 4 * sizeof(double), true) &&
@@ -585,7 +616,7 @@ tomo_status tomo_solver_create(tomo_context* ctx, const tomo_gradient_params* pr
         ok = rs_march_tex_create(ctx->hg.nx, ctx->hg.ny, ctx->hg.nz, &sv->tex) == cudaSuccess;
     if (ok && vi_texture(ctx))
         ok = rs_tex_create(ctx->hg.nu, ctx->hg.nv, ctx->hg.np, TOMO_F32, &sv->vtex, true) == cudaSuccess;
-    if (ok) sv->vi_tma = ctx->tuning.vi_layout == 2 && vi_tma_supported(ctx->g, sv->spad);
+    if (ok) sv->vi_tma = !sv->vtex.tex && vi_staged(ctx);
     if (!ok) {
         cudaGetLastError();
         tomo_solver_destroy(sv);
@@ -697,7 +728,7 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
     const double beta = sv->gg_beta;
     // dJ->addVolume(djReg, beta*lambda) with the regulariser's float lambda (GG..._CPU.cu:205).
     const float w = (float)(beta * (double)(float)P.regularization_parameter);
-    const OutView<void> resid = sv->vi_tma ? plain_view(sv->spad, h) : padded_view(sv->spad, h);
+    const OutView<void> resid = sv->vi_tma ? rows_view(sv->spad, h) : padded_view(sv->spad, h);
     const OutView<void> realv = plain_view(const_cast<void*>(real_sinogram), h);
     const bool siddon = P.projector == TOMO_PROJ_SIDDON || P.projector == TOMO_PROJ_SIDDON_REF;
     const size_t nparts = siddon ? siddon_grid_blocks(g) : rs_grid_blocks(sv->rs_layout, g);
@@ -792,8 +823,8 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
                 auto* e = tic(false);
                 if ((s = check_launch(sv->vtex.tex ? launch_vi_back_tex(um, g, sv->vtex.tex, TOMO_F32, sv->dJ, TOMO_F32, -2.0f,
                                                                         st, ctx->tuning.vi_zc)
-                                      : sv->vi_tma ? launch_vi_back_tma(um, g, (const float*)sv->spad, sv->dJ, TOMO_F32, -2.0f,
-                                                                        ctx->d_err, st)
+                                      : sv->vi_tma ? launch_vi_back_tma(um, g, (const float*)sv->spad, vi_rows_pitch(g.nu), sv->dJ,
+                                                                        TOMO_F32, -2.0f, ctx->d_err, st)
                                                    : launch_vi_back(um, g, sv->spad, TOMO_F32, sv->dJ, TOMO_F32, -2.0f, st,
                                                                     ctx->tuning.vi_zc),
                                       "vi back")) != TOMO_OK)

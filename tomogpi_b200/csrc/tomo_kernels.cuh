@@ -391,13 +391,18 @@ cudaError_t launch_ramp_filter(const void* in, tomo_dtype idt, float* out, const
 cudaError_t launch_vi_back_tex(int um, const DevGeom& g, unsigned long long tex, tomo_dtype tdt, void* vol,
                                tomo_dtype vdt, float scale, cudaStream_t st, int zc = 1);
 // VI backprojection through detector windows staged in shared memory by TMA (vi_tma.cu), of
-// an FP32 sinogram in the plain [P][nv][nu] layout: needs nu a multiple of 4 and a 16-byte
-// aligned buffer (vi_tma_supported); bounded waits report ERR_TIMEOUT in *err.
-bool vi_tma_supported(const DevGeom& g, const void* sino);
+// an FP32 sinogram [P][nv][pitch]: needs a pitch that is a multiple of 4 and a 16-byte
+// aligned buffer (vi_tma_supported); bounded waits report ERR_TIMEOUT in *err. kind: 0 VI,
+// 1 its UM variant, 2 the FDK weights.
+bool vi_tma_supported(const void* sino, long pitch);
 // stall (tests of the bounded waits only): the producer issues nothing, every consumer wait
 // runs out after its one-second bound and ERR_TIMEOUT is set.
-cudaError_t launch_vi_back_tma(int um, const DevGeom& g, const float* sino, void* vol, tomo_dtype vdt, float scale,
-                               unsigned* err, cudaStream_t st, int stall = 0);
+cudaError_t launch_vi_back_tma(int kind, const DevGeom& g, const float* sino, long pitch, void* vol, tomo_dtype vdt,
+                               float scale, unsigned* err, cudaStream_t st, int stall = 0);
+inline int vi_rows_pitch(int nu) { return (nu + 3) & ~3; }
+// Its input from a sinogram [P][nv][nu] of any type.
+cudaError_t launch_sino_rows(const void* in, tomo_dtype idt, float* out, int nu, int nv, int np, int pitch,
+                             cudaStream_t st);
 // Copies the interior of a zero-bordered padded FP32 sinogram ((nu+2) x (nv+2) per view)
 // into an FP32 layered texture of (nu, nv, np) made with a surface.
 cudaError_t tex_fill_from_padded(const float* spad, int nu, int nv, int np, const RsTexture& t, cudaStream_t st);

@@ -20,6 +20,20 @@ constexpr int vi_min_blocks(int zc) { return zc == 1 ? 5 : zc == 2 ? 2 : 1; }
 constexpr float VI_FLOOR_K = 12582912.0f;
 constexpr int VI_FLOOR_KBITS = 0x4B400000;
 
+// (1 - t) a + t b as a + t (b - a): the row and column weights enter once, so a packed lerp
+// is a subtraction (an FMA by -1, the same rounding) and an FMA.
+__device__ __forceinline__ float vi_lerp(float a, float b, float t) { return fmaf(t, fsub(b, a), a); }
+__device__ __forceinline__ float2 vi_lerp2(float2 a, float2 b, float2 t) {
+    return __ffma2_rn(t, __ffma2_rn(a, make_float2(-1.0f, -1.0f), b), a);
+}
+// Bilinear values of two samples (f32x2 lanes): texels tRC of row R, column C; column
+// weights a, row weights b.
+__device__ __forceinline__ float2 vi_bilerp2(float2 t00, float2 t10, float2 t01, float2 t11, float2 a, float2 b) {
+    return vi_lerp2(vi_lerp2(t00, t10, a), vi_lerp2(t01, t11, a), b);
+}
+
+// Positions: the reference samples its texture at u + 0.5, v + 0.5 (:403-405), whose filter
+// takes the 0.5 off again; u and v are used directly here, which saves both roundings.
 // One tile of 32 x 8 columns x (16 ZC) slices (256 threads, x fastest). Shared by the
 // single-job kernel and the batched persistent kernel (batch.cu); no block-level syncs.
 // The sixteen slices of a chunk are processed in pairs as f32x2 lanes (__fadd2_rn,
@@ -43,7 +57,7 @@ __device__ __forceinline__ void vi_tile(const DevGeom& g, const Ts* __restrict__
     const int W = g.nu + 2;
     const long VP = (long)(g.nu + 2) * (g.nv + 2);
     const float fnu = (float)g.nu, fnv = (float)g.nv;
-    const float2 MH = make_float2(-0.5f, -0.5f), K = make_float2(VI_FLOOR_K, VI_FLOOR_K);
+    const float2 K = make_float2(VI_FLOOR_K, VI_FLOOR_K);
     const float2 MK = make_float2(-VI_FLOOR_K, -VI_FLOOR_K), M1 = make_float2(-1.0f, -1.0f);
     float zp[ZC];
 #pragma unroll
@@ -58,14 +72,13 @@ __device__ __forceinline__ void vi_tile(const DevGeom& g, const Ts* __restrict__
         const float4 cv = __ldg(g.vi + p);
         float A = frcp(fadd(fadd(fmul(cv.z, xn), fmul(cv.w, yn)), g.fod));                 // :401
         const float up = fmul(fadd(fmul(cv.x, xn), fmul(cv.y, yn)), A);                  // u' (:403)
-        const float un = fadd(fadd(up, g.uc), 0.5f);
+        const float ub = fadd(up, g.uc);
         A = (p + g.p0 == 0 && !FDK) ? __double2float_rn(dmul(g.inv_gamma_d, (double)A))  // :404
                              : fmul(g.inv_gamma_f, A);                                  // :464
-        const float ub = fsub(un, 0.5f);
         if (!(ub > -1.f && ub < fnu)) continue;  // the whole column footprint is border
         const float fu = floorf(ub);
         const float a = ub - fu;
-        const float2 aa = make_float2(a, a), na = make_float2(-a, -a);
+        const float2 aa = make_float2(a, a);
         const Ts* col = spad + p * VP + ((int)fu + 1);
         float fnum = 0.f, upc = 0.f;
         if (FDK) {  // FDK3D_kernel_16reg.cuh:77-80
@@ -77,24 +90,24 @@ __device__ __forceinline__ void vi_tile(const DevGeom& g, const Ts* __restrict__
 #pragma unroll
         for (int c = 0; c < ZC; ++c) {
             float vp = fmul(A, zp[c]);                                                   // v' (:75)
-            float vn = fadd(fadd(vp, g.vc), 0.5f);                                      // :405
+            float vn = fadd(vp, g.vc);                                                   // :405
             // The chunk's rows grow with k (A > 0). When the first sample is inside the
-            // detector and vn + 16 A, an upper bound of the last one (15 rounded additions of
+            // detector and vn + 0.5 + 16 A, an upper bound of the last one (15 rounded additions of
             // values below 8192 err by less than 0.01 < A), is below nv, no sample of the chunk
             // needs the bounds test: the chunk runs without it.
-            const bool inside = !FDK && A > 0.25f && fnv <= 8192.f && fsub(vn, 0.5f) > -1.f &&
-                                fadd(vn, fmul(16.0f, A)) < fnv;
+            const bool inside = !FDK && A > 0.25f && fnv <= 8192.f && vn > -1.f &&
+                                fadd(fadd(vn, 0.5f), fmul(16.0f, A)) < fnv;
             if (FDK) {
 #pragma unroll
                 for (int k = 0; k < 16; ++k) {
-                    const float vb = fsub(vn, 0.5f);
+                    const float vb = vn;
                     if (vb > -1.f && vb < fnv) {
                         const float fv = floorf(vb);
                         const float b = vb - fv;
                         const Ts* q = col + ((int)fv + 1) * W;
-                        const float s0 = lerp(ld(q), ld(q + 1), a);
-                        const float s1 = lerp(ld(q + W), ld(q + W + 1), a);
-                        const float t = lerp(s0, s1, b);
+                        const float s0 = vi_lerp(ld(q), ld(q + 1), a);
+                        const float s1 = vi_lerp(ld(q + W), ld(q + W + 1), a);
+                        const float t = vi_lerp(s0, s1, b);
                         const float w = fdiv(fnum, fsqrt(fadd(g.fdk_beta, fadd(upc, fmul(vp, vp)))));  // :81-84
                         float& dst = (k & 1) ? acc[c][k >> 1].y : acc[c][k >> 1].x;
                         dst = fadd(dst, fmul(w, t));
@@ -107,20 +120,19 @@ __device__ __forceinline__ void vi_tile(const DevGeom& g, const Ts* __restrict__
             auto chunk = [&](auto checked) {
 #pragma unroll
                 for (int k = 0; k < 16; k += 2) {
-                    float2 vk;
+                    float2 vb;
                     if (UM) {  // v_k = v_0 + k A (_UM.cuh); the products by the scalar, never-fused
                                // multiply (a packed multiply feeding a packed add may be fused)
-                        vk = __fadd2_rn(make_float2(vn, vn), make_float2(fmul((float)k, A), fmul((float)(k + 1), A)));
+                        vb = __fadd2_rn(make_float2(vn, vn), make_float2(fmul((float)k, A), fmul((float)(k + 1), A)));
                     } else {   // v += A per slice (:410)
-                        vk.x = vn;
+                        vb.x = vn;
                         vn = fadd(vn, A);
-                        vk.y = vn;
+                        vb.y = vn;
                         vn = fadd(vn, A);
                     }
-                    const float2 vb = __fadd2_rn(vk, MH);
                     const float2 m = __fadd2_rd(vb, K);
                     const float2 f = __fadd2_rn(m, MK);
-                    const float2 b = __ffma2_rn(f, M1, vb), nb = __ffma2_rn(vb, M1, f);
+                    const float2 b = __ffma2_rn(f, M1, vb);
                     const bool ok0 = !decltype(checked)::value || (vb.x > -1.f && vb.x < fnv);
                     const bool ok1 = !decltype(checked)::value || (vb.y > -1.f && vb.y < fnv);
                     const Ts* q0 = col + (__float_as_int(m.x) - (VI_FLOOR_KBITS - 1)) * W;  // row floor + 1
@@ -129,10 +141,7 @@ __device__ __forceinline__ void vi_tile(const DevGeom& g, const Ts* __restrict__
                     const float2 t10 = make_float2(ok0 ? ld(q0 + 1) : 0.f, ok1 ? ld(q1 + 1) : 0.f);
                     const float2 t01 = make_float2(ok0 ? ld(q0 + W) : 0.f, ok1 ? ld(q1 + W) : 0.f);
                     const float2 t11 = make_float2(ok0 ? ld(q0 + W + 1) : 0.f, ok1 ? ld(q1 + W + 1) : 0.f);
-                    const float2 s0 = __ffma2_rn(aa, t10, __ffma2_rn(na, t00, t00));
-                    const float2 s1 = __ffma2_rn(aa, t11, __ffma2_rn(na, t01, t01));
-                    const float2 t = __ffma2_rn(b, s1, __ffma2_rn(nb, s0, s0));
-                    acc[c][k >> 1] = __fadd2_rn(acc[c][k >> 1], t);
+                    acc[c][k >> 1] = __fadd2_rn(acc[c][k >> 1], vi_bilerp2(t00, t10, t01, t11, aa, b));
                 }
             };
             if (inside)
@@ -180,27 +189,25 @@ __device__ __forceinline__ void vi_tile_tex(const DevGeom& g, unsigned long long
     for (int p = 0; p < g.np; ++p) {
         const float4 cv = __ldg(g.vi + p);
         float A = frcp(fadd(fadd(fmul(cv.z, xn), fmul(cv.w, yn)), g.fod));                 // :401
-        const float un = fadd(fadd(fmul(fadd(fmul(cv.x, xn), fmul(cv.y, yn)), A), g.uc), 0.5f);  // :403
+        const float ub = fadd(fmul(fadd(fmul(cv.x, xn), fmul(cv.y, yn)), A), g.uc);  // :403
         A = (p + g.p0 == 0) ? __double2float_rn(dmul(g.inv_gamma_d, (double)A))          // :404
                      : fmul(g.inv_gamma_f, A);                                          // :464
-        const float ub = fsub(un, 0.5f);
         if (!(ub > -1.f && ub < fnu)) continue;  // the whole column footprint is border
         const float fu = floorf(ub);
         const float a = ub - fu;
         const float gu = fu + 1.0f;
 #pragma unroll
         for (int c = 0; c < ZC; ++c) {
-            float vn = fadd(fadd(fmul(A, zp[c]), g.vc), 0.5f);                          // :405
+            float vn = fadd(fmul(A, zp[c]), g.vc);                                       // :405
 #pragma unroll
             for (int k = 0; k < 16; ++k) {
-                const float vk = UM ? fadd(vn, fmul((float)k, A)) : vn;
-                const float vb = fsub(vk, 0.5f);
+                const float vb = UM ? fadd(vn, fmul((float)k, A)) : vn;
                 const float fv = floorf(vb);
                 const float b = vb - fv;
                 const float4 t = gather_layer<Tt>(tex, p, gu, fv + 1.0f);
-                const float s0 = lerp(t.w, t.z, a);
-                const float s1 = lerp(t.x, t.y, a);
-                acc[c][k] = fadd(acc[c][k], lerp(s0, s1, b));
+                const float s0 = vi_lerp(t.w, t.z, a);
+                const float s1 = vi_lerp(t.x, t.y, a);
+                acc[c][k] = fadd(acc[c][k], vi_lerp(s0, s1, b));
                 if (!UM) vn = fadd(vn, A);                                              // :410
             }
         }
