@@ -1,5 +1,6 @@
-"""The forms staged in shared memory by TMA that the default tuning runs: the VI and FDK
-backprojectors (csrc/vi_tma.cu), against the forms that read global memory."""
+"""The forms staged in shared memory by TMA that the default tuning runs: the RS projector of
+FP32 volumes (csrc/rs_stage.cuh) and the VI and FDK backprojectors (csrc/vi_tma.cu), against
+the forms that read global memory."""
 import numpy as np
 import pytest
 
@@ -19,6 +20,45 @@ def _cfg(t, nx, ny, nz, nu, nv, views, pitch, mag=2.0, fod=None):
     return t.ConfigCT(fod=fod, fdd=mag * fod, projection_nb=views, u_detector_size=pitch * nu, v_detector_size=pitch * nv,
                       u_detector_pixel_nb=nu, v_detector_pixel_nb=nv, x_volume_size=float(nx), y_volume_size=float(ny),
                       z_volume_size=float(nz), x_volume_pixel_nb=nx, y_volume_pixel_nb=ny, z_volume_pixel_nb=nz)
+
+
+# (nx, ny, nz, nu, nv, views, pitch, mag[, fod]): one partial tile; odd sizes with several
+# tiles and chunks; unequal sides; pixels finer than a voxel; windows of the largest width and
+# height; too wide to stage (the texture runs); a source close enough that rays leave their
+# tile's axis; every pitch of the copies modulo 4
+RS = [(9, 7, 5, 11, 6, 5, 2.0), (101, 83, 66, 131, 95, 13, 1.9), (64, 120, 40, 97, 33, 9, 2.0),
+      (90, 90, 90, 300, 270, 7, 0.7), (120, 120, 120, 104, 108, 11, 2.4), (64, 64, 64, 20, 20, 9, 8.0),
+      (80, 80, 80, 128, 128, 12, 3.5, 2.5, 60.0), (62, 63, 61, 65, 64, 16, 2.0)]
+
+
+@pytest.mark.parametrize("kind", ["RS", "RS_UM"])
+@pytest.mark.parametrize("spec", RS, ids=lambda s: "x".join(map(str, s)))
+def test_staged_projection_equals_padded(tomo, spec, kind):
+    """Same texels, same arithmetic: bit-identical to the padded layout, in FP32 and with a
+    16-bit result; a volume of ones gives every ray its sample count in either form."""
+    cfg = _cfg(tomo, *spec)
+    vol = torch.from_numpy(np.random.default_rng(3).random(cfg.volume_shape, dtype=np.float32) + 0.25).cuda()
+    with tomo.Context(cfg) as ctx:
+        got = ctx.project(kind, vol)
+        half = ctx.project(kind, vol, dtype=torch.bfloat16)
+        ctx.set_tuning(rs_layout="plain")
+        ref = ctx.project(kind, vol)
+        torch.cuda.synchronize()
+        assert ctx.errors() == 0
+    assert float(ref.abs().max()) > 0 and torch.equal(got, ref)
+    assert torch.equal(half, ref.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("tile", [(8, 16), (16, 64), (32, 128)])
+def test_staged_projection_launch_shapes(tomo, tile):
+    """Any block shape: the windows follow the tile."""
+    cfg = _cfg(tomo, 70, 70, 50, 150, 61, 8, 1.0)
+    vol = torch.rand(cfg.volume_shape, device="cuda")
+    with tomo.Context(cfg) as ctx:
+        ctx.set_tuning(rs_warp_u=tile[0], rs_tile_u=tile[1])
+        got = ctx.project("RS", vol)
+        ctx.set_tuning(rs_layout="plain")
+        assert torch.equal(got, ctx.project("RS", vol))
 
 
 # 4, 8 and 16 slices per thread (64^3, 128^3, 160^3), partial tiles and chunks, detector

@@ -44,7 +44,7 @@ def _save():
 
 
 def size_key(cfg: ConfigCT, storage: str, gpu: str) -> str:
-    return (f"v3|{gpu}|{cfg.x_volume_pixel_nb}x{cfg.y_volume_pixel_nb}x{cfg.z_volume_pixel_nb}|"
+    return (f"v4|{gpu}|{cfg.x_volume_pixel_nb}x{cfg.y_volume_pixel_nb}x{cfg.z_volume_pixel_nb}|"
             f"{cfg.u_detector_pixel_nb}x{cfg.v_detector_pixel_nb}|{storage}")
 
 

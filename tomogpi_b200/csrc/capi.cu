@@ -53,6 +53,8 @@ struct tomo_context {
     tomo_tuning tuning{};
     int rs_in_layout[3] = {-1, -1, -1};  // layout the cached RS input buffer was sized for
     RsTexture tex;                       // TEX layout: layered array of the volume's type
+    RsStage stage;                       // TEX layout, staged: the volume's copies
+    bool stage_denied = false;           // no memory for them: the texture instead
     RsTexture vtex;                      // VI texture layout: layered array of the sinogram
     float* d_ramp = nullptr;             // ramp-filter taps for (ramp_over, ramp_cut)
     int ramp_half = 0, ramp_over = 0;
@@ -89,6 +91,7 @@ struct tomo_solver {
     int log_cap = 0;
     int next_it = 1;
     RsTexture tex;   // TEX layout resources of this solver (storage type)
+    RsStage stage;   // ... or, where the geometry allows staging, these
     RsTexture vtex;  // VI texture layout: the FP32 residual, one layer per view
     bool vi_tma = false;  // VI through TMA-staged windows: the residual is kept plain, not padded
     // host-buffer form
@@ -188,19 +191,34 @@ int effective_layout(int requested, tomo_dtype vdt, int nx, int ny, int nz) {
     return requested;
 }
 
-// Projection of a device volume into an output view (shared by tomo_project and the solver).
+// Projection of a device volume into an output view.
 tomo_status project_into(tomo_context* ctx, tomo_projector kind, const void* vol, tomo_dtype vdt, void* vpad,
                          const OutView<void>& out, tomo_dtype odt, int epi, const OutView<void>& real,
                          double* norm, cudaStream_t st) {
     const DevGeom& g = ctx->g;
     if (kind == TOMO_PROJ_RS || kind == TOMO_PROJ_RS_UM) {
         const int layout = effective_layout(ctx->tuning.rs_layout, vdt, g.nx, g.ny, g.nz);
+        if (layout == RS_LAYOUT_TEX && vdt == TOMO_F32 && !ctx->stage_denied && rs_stage_supported(g)) {
+            if (!ctx->stage.rows) {
+                const cudaError_t e = rs_stage_create(g.nx, g.ny, g.nz, &ctx->stage);
+                if (e == cudaErrorMemoryAllocation) ctx->stage_denied = true;  // the texture is half the size
+                else if (e != cudaSuccess) return cuda_fail(e, "rs stage");
+            }
+            if (!ctx->stage_denied) {
+                tomo_status s = check_launch(rs_stage_fill((const float*)vol, g.nx, g.ny, g.nz, ctx->stage, st), "rs stage fill");
+                if (s != TOMO_OK) return s;
+                return check_launch(launch_rs_stage(kind == TOMO_PROJ_RS ? 0 : 1, epi, g, ctx->stage, out, odt, real,
+                                                    TOMO_F32, norm, ctx->d_err, st),
+                                    "rs_stage_kernel");
+            }
+        }
         if (layout == RS_LAYOUT_TEX || layout == RS_LAYOUT_HYBRID || layout == RS_LAYOUT_MARCH) {
             const bool march = layout == RS_LAYOUT_MARCH;
             if (!ctx->tex.tex || ctx->tex.dt != vdt || ctx->tex.march != march) {  // the volume's type and layout
                 if (ctx->tex.tex) {
                     TOMO_CUDA_TRY(cudaStreamSynchronize(st));
                     rs_tex_destroy(&ctx->tex);
+    rs_stage_destroy(&ctx->stage);
                 }
                 cudaError_t e = march ? rs_march_tex_create(g.nx, g.ny, g.nz, &ctx->tex)
                                       : rs_vol_tex_create(g.nx, g.ny, g.nz, vdt, &ctx->tex, st);
@@ -604,12 +622,16 @@ tomo_status tomo_solver_create(tomo_context* ctx, const tomo_gradient_params* pr
         ok = alloc(&sv->vplain, ctx->nvox() * es, false);
     if (ok) {  // the norm projection's per-block partials (the launch shape is fixed by now)
         const bool sid = prm->projector == TOMO_PROJ_SIDDON || prm->projector == TOMO_PROJ_SIDDON_REF;
-        sv->npartials = sid ? siddon_grid_blocks(ctx->g) : rs_grid_blocks(sv->rs_layout, ctx->g);
+        if (!sid && sv->rs_layout == RS_LAYOUT_TEX && prm->storage == TOMO_F32 && rs_stage_supported(ctx->g) &&
+            rs_stage_create(ctx->hg.nx, ctx->hg.ny, ctx->hg.nz, &sv->stage) != cudaSuccess)
+            cudaGetLastError();  // no memory for the copies: the texture, which is half the size
+        sv->npartials = sid ? siddon_grid_blocks(ctx->g)
+                            : rs_grid_blocks(sv->stage.rows ? RS_LAYOUT_HYBRID : sv->rs_layout, ctx->g);
         // the volume norms use the same buffer (two sums of reduce_blocks partials each)
         sv->npartials = std::max(sv->npartials, 2 * reduce_blocks(ctx->hg.nx, ctx->hg.ny, ctx->hg.nz));
         ok = alloc((void**)&sv->partials, sv->npartials * sizeof(double), false);
     }
-    if (ok && (sv->rs_layout == RS_LAYOUT_TEX || sv->rs_layout == RS_LAYOUT_HYBRID))
+    if (ok && !sv->stage.rows && (sv->rs_layout == RS_LAYOUT_TEX || sv->rs_layout == RS_LAYOUT_HYBRID))
         ok = rs_vol_tex_create(ctx->hg.nx, ctx->hg.ny, ctx->hg.nz, prm->storage, &sv->tex, 0) == cudaSuccess &&
              cudaStreamSynchronize(0) == cudaSuccess;  // creation only: the zero layers are written
     if (ok && sv->rs_layout == RS_LAYOUT_MARCH)
@@ -652,6 +674,7 @@ tomo_status tomo_solver_destroy(tomo_solver* sv) {
     if (sv->ev_real) cudaEventDestroy(sv->ev_real);
     cudaFree(sv->weights);
     rs_tex_destroy(&sv->tex);
+    rs_stage_destroy(&sv->stage);
     rs_tex_destroy(&sv->vtex);
     for (auto& e : sv->ev_proj) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
     for (auto& e : sv->ev_back) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
@@ -731,7 +754,8 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
     const OutView<void> resid = sv->vi_tma ? rows_view(sv->spad, h) : padded_view(sv->spad, h);
     const OutView<void> realv = plain_view(const_cast<void*>(real_sinogram), h);
     const bool siddon = P.projector == TOMO_PROJ_SIDDON || P.projector == TOMO_PROJ_SIDDON_REF;
-    const size_t nparts = siddon ? siddon_grid_blocks(g) : rs_grid_blocks(sv->rs_layout, g);
+    const size_t nparts = siddon ? siddon_grid_blocks(g)
+                                 : rs_grid_blocks(sv->stage.rows ? RS_LAYOUT_HYBRID : sv->rs_layout, g);
     TOMO_CHECK_ARG(nparts <= sv->npartials,
                    "tomo_solver_iterate: the context's launch shape changed after the solver was created");
     // FP16 storage: max|dJ| (nrm[3] as FP32 bits) scales dJ into FP16's range before it is
@@ -751,6 +775,8 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
     // padded / cell buffer (PLAIN, CELL8, HYBRID).
     auto rs_input = [&](const float* src, const unsigned* am) -> tomo_status {
         tomo_status r;
+        if (sv->stage.rows)
+            return check_launch(rs_stage_fill(src, g.nx, g.ny, g.nz, sv->stage, st), "rs stage fill");
         if (sv->tex.tex &&
             (r = check_launch(rs_tex_fill(src, TOMO_F32, g.nx, g.ny, g.nz, sv->tex, st, am), "rs texture fill")) != TOMO_OK)
             return r;
@@ -758,6 +784,11 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
             return check_launch(launch_rs_prepare(sv->rs_layout, src, TOMO_F32, sv->vpad, sd, g.nx, g.ny, g.nz, st, am),
                                 "rs input");
         return TOMO_OK;
+    };
+    auto rs_project = [&](int epi, tomo_dtype odt, double* norm) -> cudaError_t {
+        const int um = P.projector == TOMO_PROJ_RS ? 0 : 1;
+        if (sv->stage.rows) return launch_rs_stage(um, epi, g, sv->stage, resid, odt, realv, rd, norm, ctx->d_err, st);
+        return launch_rs_project(sv->rs_layout, um, epi, g, sv->vpad, sv->tex.tex, sd, resid, odt, realv, norm, st, rd);
     };
     for (int it = first; it < first + count; ++it) {
         if (phases & TOMO_PHASE_GRADIENT) {  // residual, backprojection: dJ = -2 H^T (g - H f)
@@ -777,9 +808,7 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
                 sv->real_pending = false;
                 if ((s = rs_input(volume, nullptr)) != TOMO_OK) return s;
                 auto* e = tic(true);
-                if ((s = check_launch(launch_rs_project(sv->rs_layout, P.projector == TOMO_PROJ_RS ? 0 : 1, EPI_STORE, g,
-                                                        sv->vpad, sv->tex.tex, sd, resid, TOMO_F32, realv, nullptr, st),
-                                      "rs projection")) != TOMO_OK)
+                if ((s = check_launch(rs_project(EPI_STORE, TOMO_F32, nullptr), "rs projection")) != TOMO_OK)
                     return s;
                 toc(e);
                 TOMO_CUDA_TRY(cudaStreamWaitEvent(st, sv->ev_real, 0));
@@ -790,10 +819,7 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
             } else if (!siddon) {
                 if ((s = rs_input(volume, nullptr)) != TOMO_OK) return s;
                 auto* e = tic(true);
-                if ((s = check_launch(launch_rs_project(sv->rs_layout, P.projector == TOMO_PROJ_RS ? 0 : 1, EPI_RESIDUAL, g,
-                                                        sv->vpad, sv->tex.tex, sd,
-                                                        resid, TOMO_F32, realv, nullptr, st, rd),
-                                      "rs residual")) != TOMO_OK)
+                if ((s = check_launch(rs_project(EPI_RESIDUAL, TOMO_F32, nullptr), "rs residual")) != TOMO_OK)
                     return s;
                 toc(e);
                 sv->launches += 2;
@@ -870,10 +896,7 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
                 if (!siddon) {
                     if ((s = rs_input(sv->dJ, amax)) != TOMO_OK) return s;
                     auto* e = tic(true);
-                    if ((s = check_launch(launch_rs_project(sv->rs_layout, P.projector == TOMO_PROJ_RS ? 0 : 1, EPI_NORM, g,
-                                                            sv->vpad, sv->tex.tex, sd,
-                                                            resid, sd, realv, sv->partials, st),
-                                          "rs norm")) != TOMO_OK)
+                    if ((s = check_launch(rs_project(EPI_NORM, sd, sv->partials), "rs norm")) != TOMO_OK)
                         return s;
                     toc(e);
                     sv->launches += 2;

@@ -14,16 +14,16 @@ namespace tomo {
 // One trilinear sample, sm_100 packed FP32.
 //
 // The reference samples tex3D at t = P + 0.5 (P the ray position, projection_ER_kernel.cuh
-// :292) and the exact-FP32 filter reads the texels around v = t - 0.5 with weights
-// v - floor(v). Both roundings are kept (t and v are computed as written); the floors are
-// exact: adding 1.5 * 2^23 with rounding toward -inf gives floor(v) + 1.5 * 2^23 exactly for
-// |v| < 2^22 (the spacing of floats in [2^23, 2^24) is 1), so the float floor is that sum
-// minus the constant and the integer floor is its bit pattern minus the constant's. This
-// keeps every floor and conversion off the XU pipe, and the x / y (and duplicated z)
-// coordinates run as f32x2 pairs (__fadd2_rn, __ffma2_rn round each lane like the scalar
-// operation). Every layout interpolates the same way: first between the two slices (two
-// packed lerps over the four texel columns), then along x, then along y, so all layouts
-// give bit-identical sums.
+// :292) and the filter reads the texels around t - 0.5: P itself is used here, which saves
+// both roundings (and four packed additions a sample). The floors are exact: adding
+// 1.5 * 2^23 with rounding toward -inf gives floor(v) + 1.5 * 2^23 exactly for |v| < 2^22
+// (the spacing of floats in [2^23, 2^24) is 1), so the float floor is that sum minus the
+// constant and the integer floor is its bit pattern minus the constant's. This keeps every
+// floor and conversion off the XU pipe. The x / y coordinates run as f32x2 pairs
+// (__fadd2_rn, __ffma2_rn round each lane like the scalar operation), z as a scalar: a
+// packed operation holds the FMA pipe for two. Every layout interpolates the same way:
+// first between the two slices (two packed lerps over the four texel columns), then along
+// x, then along y, so all layouts give bit-identical sums.
 // ---------------------------------------------------------------------------------
 constexpr float FLOOR_K = 12582912.0f;   // 1.5 * 2^23
 constexpr int FLOOR_KBITS = 0x4B400000;  // its bit pattern
@@ -38,24 +38,22 @@ struct RsSample {
     int ix, iy, iz; // floor + FLOOR_KBITS, as integers
 };
 
-__device__ __forceinline__ RsSample rs_sample(float2 AB, float2 CC) {
-    const float2 H = make_float2(0.5f, 0.5f), MH = make_float2(-0.5f, -0.5f);
+__device__ __forceinline__ RsSample rs_sample(float2 AB, float C) {
     const float2 K = make_float2(FLOOR_K, FLOOR_K), MK = make_float2(-FLOOR_K, -FLOOR_K);
-    const float2 M1 = make_float2(-1.0f, -1.0f);
     RsSample s;
-    s.v = __fadd2_rn(__fadd2_rn(AB, H), MH);
-    const float2 vzz = __fadd2_rn(__fadd2_rn(CC, H), MH);
-    s.vz = vzz.x;
-    const float2 m = __fadd2_rd(s.v, K), mz = __fadd2_rd(vzz, K);
+    s.v = AB;
+    s.vz = C;
+    const float2 m = __fadd2_rd(AB, K);
+    const float mz = __fadd_rd(C, FLOOR_K);
     s.f = __fadd2_rn(m, MK);
-    const float2 fz = __fadd2_rn(mz, MK);
-    s.fz = fz.x;
-    s.w = __ffma2_rn(s.f, M1, s.v);
-    s.cc = __ffma2_rn(fz, M1, vzz);
-    s.ncc = __ffma2_rn(vzz, M1, fz);
+    s.fz = fsub(mz, FLOOR_K);
+    s.w = __ffma2_rn(s.f, make_float2(-1.0f, -1.0f), AB);
+    const float c = fsub(C, s.fz);
+    s.cc = make_float2(c, c);
+    s.ncc = make_float2(-c, -c);
     s.ix = __float_as_int(m.x);
     s.iy = __float_as_int(m.y);
-    s.iz = __float_as_int(mz.x);
+    s.iz = __float_as_int(mz);
     return s;
 }
 
@@ -366,14 +364,15 @@ __device__ __forceinline__ void rs_tile(const DevGeom& g, const Tv* __restrict__
         if (hit) {
             const float fnx = (float)g.nx, fny = (float)g.ny, fnz = (float)g.nz;
             const float dx = g.dx;
-            const float2 SXY = make_float2(r.sx, r.sy), SZZ = make_float2(r.sz, r.sz);
+            const float2 SXY = make_float2(r.sx, r.sy);
             auto march = [&](auto sample) {
-                float2 AB = make_float2(r.A, r.B), CC = make_float2(r.C, r.C);
+                float2 AB = make_float2(r.A, r.B);
+                float C = r.C;
                 for (unsigned n = 0; n < r.n; ++n) {
-                    const RsSample s = rs_sample(AB, CC);
+                    const RsSample s = rs_sample(AB, C);
                     acc = fadd(acc, fmul(dx, sample(s, n)));  // :292
                     AB = __fadd2_rn(AB, SXY);              // :295-297
-                    CC = __fadd2_rn(CC, SZZ);
+                    C = fadd(C, r.sz);
                 }
             };
             if (LAYOUT == RS_LAYOUT_MARCH) {

@@ -17,7 +17,9 @@
 //          eight texels stored together: 32 B (FP32) or 16 B (BF16/FP16), aligned, so a
 //          sample is two (one) 128-bit loads from a single sector. 8x the volume's bytes.
 //   TEX    2D layered array in the storage type (raw 16-bit for BF16/FP16), slice z in
-//          layer z + 1 between two zero layers; two 4-texel tld4 gathers per sample.
+//          layer z + 1 between two zero layers; two 4-texel tld4 gathers per sample. FP32
+//          volumes are staged in shared memory instead where the geometry allows it
+//          (rs_stage.cuh; this texture when it does not, or without memory for the copies).
 //   HYBRID TEX for the lower slice of a sample plus, for the upper slice, quads (the slice's
 //          four footprint texels in tld4 order, 16 B FP32 / 8 B 16-bit) in global memory, in a
 //          row-major and a column-major array: one gather and one 128-bit load per sample.
@@ -160,10 +162,9 @@ __global__ void __launch_bounds__(256) rs_adjoint_kernel(DevGeom g, const Ts* __
     const float fnx = (float)g.nx, fny = (float)g.ny, fnz = (float)g.nz;
     float A = r.A, B = r.B, C = r.C;
     for (unsigned n = 0; n < r.n; ++n) {
-        const float xb = fsub(fadd(A, 0.5f), 0.5f), yb = fsub(fadd(B, 0.5f), 0.5f), zb = fsub(fadd(C, 0.5f), 0.5f);
-        if (xb > -1.f && yb > -1.f && zb > -1.f && xb < fnx && yb < fny && zb < fnz) {
-            const float fx = floorf(xb), fy = floorf(yb), fz = floorf(zb);
-            const float a = xb - fx, b = yb - fy, c = zb - fz;
+        if (A > -1.f && B > -1.f && C > -1.f && A < fnx && B < fny && C < fnz) {
+            const float fx = floorf(A), fy = floorf(B), fz = floorf(C);
+            const float a = A - fx, b = B - fy, c = C - fz;
             const int i = (int)fx, j = (int)fy, k = (int)fz;
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
