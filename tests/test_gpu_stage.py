@@ -49,6 +49,34 @@ def test_staged_projection_equals_padded(tomo, spec, kind):
     assert torch.equal(half, ref.to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("storage", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("spec", [(128, 128, 128, 128, 128, 45, 2.0), (131, 127, 130, 150, 141, 33, 1.7)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_half_staged_projection_equals_cells(tomo, spec, storage):
+    """16-bit volumes from 128^3 on: some blocks stage slice pairs, the others gather them from
+    the texture; bit-identical to the cell layout, from 16-bit volumes and, in the solver, from
+    an FP32 iterate converted on the way (one iteration)."""
+    cfg = _cfg(tomo, *spec)
+    vol = torch.from_numpy(np.random.default_rng(8).random(cfg.volume_shape, dtype=np.float32)).cuda()
+    real = torch.rand(cfg.sinogram_shape, device="cuda")
+    par = tomo.GradientParams(gradient_iteration_nb=1, optimal_step_iteration_nb=2, real_f32=True,
+                              storage="bf16" if storage == torch.bfloat16 else "f16")
+    out = {}
+    for lay in ("tex", "cell8"):
+        with tomo.Context(cfg) as ctx:
+            ctx.set_tuning(rs_layout=lay)
+            out[lay] = [ctx.project(k, vol.to(storage), dtype=torch.float32) for k in ("RS", "RS_UM")]
+            f = vol.clone()
+            tomo.Solver(ctx, par).iterate(f, real)
+            out[lay].append(f)  # the step's norm is summed per block: FP64 sums in another order
+            torch.cuda.synchronize()
+            assert ctx.errors() == 0
+    for a, b in zip(out["tex"][:2], out["cell8"][:2]):
+        assert float(b.abs().max()) > 0 and torch.equal(a, b)
+    a, b = out["tex"][2], out["cell8"][2]
+    assert float(torch.linalg.vector_norm((a - b).double()) / torch.linalg.vector_norm(b.double())) <= 1e-6
+
+
 @pytest.mark.parametrize("tile", [(8, 16), (16, 64), (32, 128)])
 def test_staged_projection_launch_shapes(tomo, tile):
     """Any block shape: the windows follow the tile."""

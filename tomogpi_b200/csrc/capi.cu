@@ -132,6 +132,34 @@ tomo_status ensure(void** p, size_t bytes, bool zero) {
     return TOMO_OK;
 }
 
+// The same for a context's or solver's buffers: its staged copies give way to them (its
+// projections then gather from the texture, half the size in FP32).
+tomo_status ensure_beside(RsStage* stage, void** p, size_t bytes, bool zero) {
+    const tomo_status s = ensure(p, bytes, zero);
+    if (s != TOMO_ERR_NO_MEMORY || !stage->rows) return s;
+    cudaGetLastError();
+    TOMO_CUDA_TRY(cudaDeviceSynchronize());
+    rs_stage_destroy(stage);
+    return ensure(p, bytes, zero);
+}
+tomo_status ensure(tomo_context* ctx, void** p, size_t bytes, bool zero) {
+    const bool staged = ctx->stage.rows != nullptr;
+    const tomo_status s = ensure_beside(&ctx->stage, p, bytes, zero);
+    if (staged && !ctx->stage.rows) ctx->stage_denied = true;
+    return s;
+}
+cudaError_t solver_texture(tomo_solver* sv) {
+    const HostGeom& h = sv->ctx->hg;
+    const cudaError_t e = rs_vol_tex_create(h.nx, h.ny, h.nz, sv->prm.storage, &sv->tex, 0);
+    return e == cudaSuccess ? cudaStreamSynchronize(0) : e;  // creation only: the zero layers are written
+}
+tomo_status ensure(tomo_solver* sv, void** p, size_t bytes, bool zero) {
+    const bool staged = sv->stage.rows != nullptr;
+    const tomo_status s = ensure_beside(&sv->stage, p, bytes, zero);
+    if (staged && !sv->stage.rows && !sv->tex.tex) TOMO_CUDA_TRY(solver_texture(sv));
+    return s;
+}
+
 tomo_status set_device(const tomo_context* ctx) {
     TOMO_CUDA_TRY(cudaSetDevice(ctx->device));
     cudaGetLastError();  // drop a stale non-sticky error so launch checks report their own
@@ -191,6 +219,22 @@ int effective_layout(int requested, tomo_dtype vdt, int nx, int ny, int nz) {
     return requested;
 }
 
+// The context's texture for a volume of type vdt (MARCH: its even faces), created or replaced
+// where it is of another kind, filled from the volume.
+tomo_status context_texture(tomo_context* ctx, bool march, const void* vol, tomo_dtype vdt, cudaStream_t st) {
+    const DevGeom& g = ctx->g;
+    if (!ctx->tex.tex || ctx->tex.dt != vdt || ctx->tex.march != march) {
+        if (ctx->tex.tex) {
+            TOMO_CUDA_TRY(cudaStreamSynchronize(st));
+            rs_tex_destroy(&ctx->tex);
+        }
+        const cudaError_t e = march ? rs_march_tex_create(g.nx, g.ny, g.nz, &ctx->tex)
+                                    : rs_vol_tex_create(g.nx, g.ny, g.nz, vdt, &ctx->tex, st);
+        if (e != cudaSuccess) return cuda_fail(e, "rs texture");
+    }
+    return check_launch(rs_tex_fill(vol, vdt, g.nx, g.ny, g.nz, ctx->tex, st), "rs texture fill");
+}
+
 // Projection of a device volume into an output view.
 tomo_status project_into(tomo_context* ctx, tomo_projector kind, const void* vol, tomo_dtype vdt, void* vpad,
                          const OutView<void>& out, tomo_dtype odt, int epi, const OutView<void>& real,
@@ -198,34 +242,32 @@ tomo_status project_into(tomo_context* ctx, tomo_projector kind, const void* vol
     const DevGeom& g = ctx->g;
     if (kind == TOMO_PROJ_RS || kind == TOMO_PROJ_RS_UM) {
         const int layout = effective_layout(ctx->tuning.rs_layout, vdt, g.nx, g.ny, g.nz);
-        if (layout == RS_LAYOUT_TEX && vdt == TOMO_F32 && !ctx->stage_denied && rs_stage_supported(g)) {
-            if (!ctx->stage.rows) {
-                const cudaError_t e = rs_stage_create(g.nx, g.ny, g.nz, &ctx->stage);
-                if (e == cudaErrorMemoryAllocation) ctx->stage_denied = true;  // the texture is half the size
-                else if (e != cudaSuccess) return cuda_fail(e, "rs stage");
+        bool staged = layout == RS_LAYOUT_TEX && !ctx->stage_denied && rs_stage_supported(g, vdt);
+        if (layout == RS_LAYOUT_HYBRID || layout == RS_LAYOUT_MARCH || (layout == RS_LAYOUT_TEX && !(staged && vdt == TOMO_F32))) {
+            const tomo_status s = context_texture(ctx, layout == RS_LAYOUT_MARCH, vol, vdt, st);
+            if (s != TOMO_OK) return s;
+        }
+        if (staged) {
+            if (ctx->stage.rows && ctx->stage.dt != vdt) {
+                TOMO_CUDA_TRY(cudaStreamSynchronize(st));
+                rs_stage_destroy(&ctx->stage);
             }
-            if (!ctx->stage_denied) {
-                tomo_status s = check_launch(rs_stage_fill((const float*)vol, g.nx, g.ny, g.nz, ctx->stage, st), "rs stage fill");
+            cudaError_t e = ctx->stage.rows ? cudaSuccess : rs_stage_create(g.nx, g.ny, g.nz, vdt, &ctx->stage);
+            if (e == cudaErrorMemoryAllocation) {  // no memory for the copies: the texture alone
+                ctx->stage_denied = true;
+                staged = false;
+                const tomo_status s = vdt == TOMO_F32 ? context_texture(ctx, false, vol, vdt, st) : TOMO_OK;
                 if (s != TOMO_OK) return s;
-                return check_launch(launch_rs_stage(kind == TOMO_PROJ_RS ? 0 : 1, epi, g, ctx->stage, out, odt, real,
-                                                    TOMO_F32, norm, ctx->d_err, st),
-                                    "rs_stage_kernel");
+            } else if (e != cudaSuccess) {
+                return cuda_fail(e, "rs stage");
             }
         }
-        if (layout == RS_LAYOUT_TEX || layout == RS_LAYOUT_HYBRID || layout == RS_LAYOUT_MARCH) {
-            const bool march = layout == RS_LAYOUT_MARCH;
-            if (!ctx->tex.tex || ctx->tex.dt != vdt || ctx->tex.march != march) {  // the volume's type and layout
-                if (ctx->tex.tex) {
-                    TOMO_CUDA_TRY(cudaStreamSynchronize(st));
-                    rs_tex_destroy(&ctx->tex);
-    rs_stage_destroy(&ctx->stage);
-                }
-                cudaError_t e = march ? rs_march_tex_create(g.nx, g.ny, g.nz, &ctx->tex)
-                                      : rs_vol_tex_create(g.nx, g.ny, g.nz, vdt, &ctx->tex, st);
-                if (e != cudaSuccess) return cuda_fail(e, "rs texture");
-            }
-            if (check_launch(rs_tex_fill(vol, vdt, g.nx, g.ny, g.nz, ctx->tex, st), "rs texture fill") != TOMO_OK)
-                return TOMO_ERR_CUDA;
+        if (staged) {
+            const tomo_status s = check_launch(rs_stage_fill(vol, vdt, g.nx, g.ny, g.nz, ctx->stage, st), "rs stage fill");
+            if (s != TOMO_OK) return s;
+            return check_launch(launch_rs_stage(kind == TOMO_PROJ_RS ? 0 : 1, epi, g, ctx->stage, ctx->tex.tex, out, odt, real,
+                                                TOMO_F32, norm, ctx->d_err, st),
+                                "rs_stage_kernel");
         }
         if (layout != RS_LAYOUT_TEX &&  // HYBRID: the texture above plus its cell buffer
             check_launch(launch_rs_prepare(layout, vol, vdt, vpad, vdt, g.nx, g.ny, g.nz, st), "rs input") != TOMO_OK)
@@ -388,7 +430,7 @@ tomo_status tomo_project(tomo_context* ctx, tomo_projector kind, const void* vol
             cudaFree(ctx->vpad[volume_dtype]);
             ctx->vpad[volume_dtype] = nullptr;
         }
-        s = ensure(&ctx->vpad[volume_dtype], rs_input_elems(layout, ctx->hg.nx, ctx->hg.ny, ctx->hg.nz) *
+        s = ensure(ctx, &ctx->vpad[volume_dtype], rs_input_elems(layout, ctx->hg.nx, ctx->hg.ny, ctx->hg.nz) *
                                                  dtype_size(volume_dtype), true);
         if (s != TOMO_OK) return s;
         ctx->rs_in_layout[volume_dtype] = layout;
@@ -445,7 +487,7 @@ tomo_status tomo_backproject(tomo_context* ctx, tomo_backprojector kind, const v
                                 "vi_back_tma_kernel");
     }
     if (kind == TOMO_BACK_FDK) {
-        s = ensure(&ctx->spad[sinogram_dtype], ctx->nsino_pad() * dtype_size(sinogram_dtype), true);
+        s = ensure(ctx, &ctx->spad[sinogram_dtype], ctx->nsino_pad() * dtype_size(sinogram_dtype), true);
         if (s != TOMO_OK) return s;
         void* sp = ctx->spad[sinogram_dtype];
         if ((s = check_launch(launch_pad_sinogram(sinogram, sinogram_dtype, sp, sinogram_dtype, g.nu, g.nv, g.np, st),
@@ -454,7 +496,7 @@ tomo_status tomo_backproject(tomo_context* ctx, tomo_backprojector kind, const v
         return check_launch(launch_vi_fdk(g, sp, sinogram_dtype, volume, volume_dtype, st), "vi_back_kernel (FDK)");
     }
     if (kind == TOMO_BACK_VI || kind == TOMO_BACK_VI_UM) {
-        s = ensure(&ctx->spad[sinogram_dtype], ctx->nsino_pad() * dtype_size(sinogram_dtype), true);
+        s = ensure(ctx, &ctx->spad[sinogram_dtype], ctx->nsino_pad() * dtype_size(sinogram_dtype), true);
         if (s != TOMO_OK) return s;
         void* sp = ctx->spad[sinogram_dtype];
         if ((s = check_launch(launch_pad_sinogram(sinogram, sinogram_dtype, sp, sinogram_dtype, g.nu, g.nv, g.np, st),
@@ -467,7 +509,7 @@ tomo_status tomo_backproject(tomo_context* ctx, tomo_backprojector kind, const v
     // Matched transposes: FP32 scatter, converted if the output is 16-bit.
     float* acc = (float*)volume;
     if (volume_dtype != TOMO_F32) {
-        s = ensure((void**)&ctx->adj_scratch, ctx->nvox() * sizeof(float), false);
+        s = ensure(ctx, (void**)&ctx->adj_scratch, ctx->nvox() * sizeof(float), false);
         if (s != TOMO_OK) return s;
         acc = ctx->adj_scratch;
     }
@@ -514,8 +556,8 @@ tomo_status tomo_ramp_filter_host(tomo_context* ctx, const float* sinogram, floa
     std::lock_guard<std::mutex> lock(ctx->mu);
     tomo_status s = set_device(ctx);
     if (s != TOMO_OK) return s;
-    if ((s = ensure(&ctx->spad[TOMO_F32], ctx->nsino_pad() * sizeof(float), true)) != TOMO_OK) return s;
-    if ((s = ensure((void**)&ctx->h_sino, ctx->nsino() * sizeof(float), false)) != TOMO_OK) return s;
+    if ((s = ensure(ctx, &ctx->spad[TOMO_F32], ctx->nsino_pad() * sizeof(float), true)) != TOMO_OK) return s;
+    if ((s = ensure(ctx, (void**)&ctx->h_sino, ctx->nsino() * sizeof(float), false)) != TOMO_OK) return s;
     cudaStream_t st = ctx->host_stream;
     float* filt = (float*)ctx->spad[TOMO_F32];  // scratch of at least nsino floats
     TOMO_CUDA_TRY(cudaMemcpyAsync(ctx->h_sino, sinogram, ctx->nsino() * sizeof(float), cudaMemcpyHostToDevice, st));
@@ -530,8 +572,8 @@ tomo_status tomo_project_host(tomo_context* ctx, tomo_projector kind, const floa
     std::lock_guard<std::mutex> lock(ctx->mu);
     tomo_status s = set_device(ctx);
     if (s != TOMO_OK) return s;
-    if ((s = ensure((void**)&ctx->h_vol, ctx->nvox() * sizeof(float), false)) != TOMO_OK) return s;
-    if ((s = ensure((void**)&ctx->h_sino, ctx->nsino() * sizeof(float), false)) != TOMO_OK) return s;
+    if ((s = ensure(ctx, (void**)&ctx->h_vol, ctx->nvox() * sizeof(float), false)) != TOMO_OK) return s;
+    if ((s = ensure(ctx, (void**)&ctx->h_sino, ctx->nsino() * sizeof(float), false)) != TOMO_OK) return s;
     cudaStream_t st = ctx->host_stream;
     TOMO_CUDA_TRY(cudaMemcpyAsync(ctx->h_vol, volume, ctx->nvox() * sizeof(float), cudaMemcpyHostToDevice, st));
     if ((s = tomo_project(ctx, kind, ctx->h_vol, TOMO_F32, ctx->h_sino, TOMO_F32, st)) != TOMO_OK) return s;
@@ -545,8 +587,8 @@ tomo_status tomo_backproject_host(tomo_context* ctx, tomo_backprojector kind, co
     std::lock_guard<std::mutex> lock(ctx->mu);
     tomo_status s = set_device(ctx);
     if (s != TOMO_OK) return s;
-    if ((s = ensure((void**)&ctx->h_vol, ctx->nvox() * sizeof(float), false)) != TOMO_OK) return s;
-    if ((s = ensure((void**)&ctx->h_sino, ctx->nsino() * sizeof(float), false)) != TOMO_OK) return s;
+    if ((s = ensure(ctx, (void**)&ctx->h_vol, ctx->nvox() * sizeof(float), false)) != TOMO_OK) return s;
+    if ((s = ensure(ctx, (void**)&ctx->h_sino, ctx->nsino() * sizeof(float), false)) != TOMO_OK) return s;
     cudaStream_t st = ctx->host_stream;
     TOMO_CUDA_TRY(cudaMemcpyAsync(ctx->h_sino, sinogram, ctx->nsino() * sizeof(float), cudaMemcpyHostToDevice, st));
     if ((s = tomo_backproject(ctx, kind, ctx->h_sino, TOMO_F32, ctx->h_vol, TOMO_F32, st)) != TOMO_OK) return s;
@@ -620,25 +662,29 @@ tomo_status tomo_solver_create(tomo_context* ctx, const tomo_gradient_params* pr
               alloc((void**)&sv->alpha_log, sv->log_cap * sizeof(double), true);
     if (ok && prm->storage != TOMO_F32 && (prm->projector == TOMO_PROJ_SIDDON || prm->projector == TOMO_PROJ_SIDDON_REF))
         ok = alloc(&sv->vplain, ctx->nvox() * es, false);
+    const bool rs = prm->projector == TOMO_PROJ_RS || prm->projector == TOMO_PROJ_RS_UM;
+    const bool staged = rs && sv->rs_layout == RS_LAYOUT_TEX && rs_stage_supported(ctx->g, prm->storage);
+    if (ok && !(staged && prm->storage == TOMO_F32) &&
+        (sv->rs_layout == RS_LAYOUT_TEX || sv->rs_layout == RS_LAYOUT_HYBRID))
+        ok = solver_texture(sv) == cudaSuccess;
     if (ok) {  // the norm projection's per-block partials (the launch shape is fixed by now)
         const bool sid = prm->projector == TOMO_PROJ_SIDDON || prm->projector == TOMO_PROJ_SIDDON_REF;
-        if (!sid && sv->rs_layout == RS_LAYOUT_TEX && prm->storage == TOMO_F32 && rs_stage_supported(ctx->g) &&
-            rs_stage_create(ctx->hg.nx, ctx->hg.ny, ctx->hg.nz, &sv->stage) != cudaSuccess)
-            cudaGetLastError();  // no memory for the copies: the texture, which is half the size
-        sv->npartials = sid ? siddon_grid_blocks(ctx->g)
-                            : rs_grid_blocks(sv->stage.rows ? RS_LAYOUT_HYBRID : sv->rs_layout, ctx->g);
+        sv->npartials = sid ? siddon_grid_blocks(ctx->g) : rs_grid_blocks(sv->rs_layout, ctx->g);
+        if (staged) sv->npartials = std::max(sv->npartials, rs_stage_grid_blocks(ctx->g));
         // the volume norms use the same buffer (two sums of reduce_blocks partials each)
         sv->npartials = std::max(sv->npartials, 2 * reduce_blocks(ctx->hg.nx, ctx->hg.ny, ctx->hg.nz));
         ok = alloc((void**)&sv->partials, sv->npartials * sizeof(double), false);
     }
-    if (ok && !sv->stage.rows && (sv->rs_layout == RS_LAYOUT_TEX || sv->rs_layout == RS_LAYOUT_HYBRID))
-        ok = rs_vol_tex_create(ctx->hg.nx, ctx->hg.ny, ctx->hg.nz, prm->storage, &sv->tex, 0) == cudaSuccess &&
-             cudaStreamSynchronize(0) == cudaSuccess;  // creation only: the zero layers are written
     if (ok && sv->rs_layout == RS_LAYOUT_MARCH)
         ok = rs_march_tex_create(ctx->hg.nx, ctx->hg.ny, ctx->hg.nz, &sv->tex) == cudaSuccess;
     if (ok && vi_texture(ctx))
         ok = rs_tex_create(ctx->hg.nu, ctx->hg.nv, ctx->hg.np, TOMO_F32, &sv->vtex, true) == cudaSuccess;
     if (ok) sv->vi_tma = !sv->vtex.tex && vi_staged(ctx);
+    // last, and given back when a later allocation needs the room (ensure)
+    if (ok && staged && rs_stage_create(ctx->hg.nx, ctx->hg.ny, ctx->hg.nz, prm->storage, &sv->stage) != cudaSuccess) {
+        cudaGetLastError();  // no memory for the copies: the texture alone
+        ok = sv->tex.tex || solver_texture(sv) == cudaSuccess;
+    }
     if (!ok) {
         cudaGetLastError();
         tomo_solver_destroy(sv);
@@ -690,7 +736,7 @@ tomo_status tomo_solver_set_regularizer(tomo_solver* sv, int32_t kind, double hu
                    "tomo_solver_set_regularizer: the Huber threshold must be finite and non-negative");
     if (kind == TOMO_REG_HUBER && !sv->htmp) {
         TOMO_CUDA_TRY(cudaSetDevice(sv->device));
-        if (cudaMalloc((void**)&sv->htmp, sv->ctx->nvox() * sizeof(float)) != cudaSuccess) {
+        if (ensure(sv, (void**)&sv->htmp, sv->ctx->nvox() * sizeof(float), false) != TOMO_OK) {
             cudaGetLastError();
             sv->htmp = nullptr;
             set_error("tomo_solver_set_regularizer: device allocation failed");
@@ -717,7 +763,7 @@ tomo_status tomo_solver_set_weights(tomo_solver* sv, const float* weights, int32
     cudaStream_t st = (cudaStream_t)stream;
     if (weights) {  // Iter3D_Algo_Gradient.cu:243-248: the loop holds its own weight sinogram
         const size_t bytes = sv->ctx->nsino() * sizeof(float);
-        if ((s = ensure((void**)&sv->weights, bytes, false)) != TOMO_OK) return s;
+        if ((s = ensure(sv, (void**)&sv->weights, bytes, false)) != TOMO_OK) return s;
         if (host) {
             TOMO_CUDA_TRY(cudaMemcpy(sv->weights, weights, bytes, cudaMemcpyHostToDevice));
         } else {
@@ -754,8 +800,9 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
     const OutView<void> resid = sv->vi_tma ? rows_view(sv->spad, h) : padded_view(sv->spad, h);
     const OutView<void> realv = plain_view(const_cast<void*>(real_sinogram), h);
     const bool siddon = P.projector == TOMO_PROJ_SIDDON || P.projector == TOMO_PROJ_SIDDON_REF;
-    const size_t nparts = siddon ? siddon_grid_blocks(g)
-                                 : rs_grid_blocks(sv->stage.rows ? RS_LAYOUT_HYBRID : sv->rs_layout, g);
+    const size_t nparts = siddon           ? siddon_grid_blocks(g)
+                          : sv->stage.rows ? rs_stage_grid_blocks(g)
+                                           : rs_grid_blocks(sv->rs_layout, g);
     TOMO_CHECK_ARG(nparts <= sv->npartials,
                    "tomo_solver_iterate: the context's launch shape changed after the solver was created");
     // FP16 storage: max|dJ| (nrm[3] as FP32 bits) scales dJ into FP16's range before it is
@@ -775,8 +822,9 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
     // padded / cell buffer (PLAIN, CELL8, HYBRID).
     auto rs_input = [&](const float* src, const unsigned* am) -> tomo_status {
         tomo_status r;
-        if (sv->stage.rows)
-            return check_launch(rs_stage_fill(src, g.nx, g.ny, g.nz, sv->stage, st), "rs stage fill");
+        if (sv->stage.rows &&
+            (r = check_launch(rs_stage_fill(src, TOMO_F32, g.nx, g.ny, g.nz, sv->stage, st, am), "rs stage fill")) != TOMO_OK)
+            return r;
         if (sv->tex.tex &&
             (r = check_launch(rs_tex_fill(src, TOMO_F32, g.nx, g.ny, g.nz, sv->tex, st, am), "rs texture fill")) != TOMO_OK)
             return r;
@@ -787,7 +835,7 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
     };
     auto rs_project = [&](int epi, tomo_dtype odt, double* norm) -> cudaError_t {
         const int um = P.projector == TOMO_PROJ_RS ? 0 : 1;
-        if (sv->stage.rows) return launch_rs_stage(um, epi, g, sv->stage, resid, odt, realv, rd, norm, ctx->d_err, st);
+        if (sv->stage.rows) return launch_rs_stage(um, epi, g, sv->stage, sv->tex.tex, resid, odt, realv, rd, norm, ctx->d_err, st);
         return launch_rs_project(sv->rs_layout, um, epi, g, sv->vpad, sv->tex.tex, sd, resid, odt, realv, norm, st, rd);
     };
     for (int it = first; it < first + count; ++it) {
@@ -970,8 +1018,8 @@ tomo_status tomo_solver_iterate_host(tomo_solver* sv, float* volume, const void*
     if (s != TOMO_OK) return s;
     cudaStream_t st = (cudaStream_t)stream;
     const size_t rb = ctx->nsino() * dtype_size(sv->prm.real_sinogram_f32 ? TOMO_F32 : sv->prm.storage);
-    if ((s = ensure((void**)&sv->d_vol, ctx->nvox() * sizeof(float), false)) != TOMO_OK) return s;
-    if ((s = ensure(&sv->d_real, rb, false)) != TOMO_OK) return s;
+    if ((s = ensure(sv, (void**)&sv->d_vol, ctx->nvox() * sizeof(float), false)) != TOMO_OK) return s;
+    if ((s = ensure(sv, &sv->d_real, rb, false)) != TOMO_OK) return s;
     TOMO_CUDA_TRY(cudaMemcpyAsync(sv->d_vol, volume, ctx->nvox() * sizeof(float), cudaMemcpyHostToDevice, st));
     const bool siddon = sv->prm.projector == TOMO_PROJ_SIDDON || sv->prm.projector == TOMO_PROJ_SIDDON_REF;
     if (!siddon && count > 0) {

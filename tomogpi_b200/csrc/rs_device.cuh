@@ -345,7 +345,7 @@ __device__ __forceinline__ bool rs_ray_inside(const DevGeom& g, const RsRay& r) 
 // One 2^rs_tlog u x 2^(8 - rs_tlog) v tile of view p (256 threads; each warp's rays span
 // 2^rs_wlog u x 2^(5 - rs_wlog) v): ray set-up,
 // trilinear march, epilogue. Shared by the single-job kernel and the batched persistent
-// kernel (batch.cu); must be called by all 256 threads of the block (EPI_NORM syncs).
+// kernel (batch.cu); must be called by all threads of the block (EPI_NORM syncs).
 template <int MODE, int LAYOUT, typename Tv, typename To, int EPI, typename Tr = To>
 __device__ __forceinline__ void rs_tile(const DevGeom& g, const Tv* __restrict__ vin, unsigned long long tex,
                                         const OutView<To>& out, const OutView<Tr>& real, double* __restrict__ norm,
@@ -355,7 +355,7 @@ __device__ __forceinline__ void rs_tile(const DevGeom& g, const Tv* __restrict__
     const int wpr = 1 << (g.rs_tlog - wl);               // warps per row of the tile
     const int u = (ut << g.rs_tlog) + (warp & (wpr - 1)) * wu + (lane & (wu - 1));
     const int v = vt * rs_tile_v(g) + (warp >> (g.rs_tlog - wl)) * (32 >> wl) + (lane >> wl);
-    const bool active = (u < g.nu) && (v < g.nv);
+    const bool active = warp < 8 && (u < g.nu) && (v < g.nv);  // (a staged block has a ninth warp)
     float acc = 0.f;
     if (active) {
         RsRay r;

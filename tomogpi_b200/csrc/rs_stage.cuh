@@ -2,15 +2,16 @@
 // of the volume that a block's rays cross is brought into shared memory by the Tensor
 // Memory Accelerator (TMA), a few planes at a time, while the rays march through it.
 //
-// FP32 volumes. What bounds the other FP32 layouts is the L1TEX unit: a texture gather
-// returns 32 B a clock and SM, so each of a TEX sample's two gathers takes it 16 clocks per
-// warp, whatever the cache hit rate. Shared memory returns 128 B a clock: a sample's eight
-// 32-bit reads take 15.9 clocks per warp with their bank conflicts (the 32 lanes' texels lie
-// in a patch of about 40 words, so two lanes of some bank usually differ). Neighbouring rays
-// share texels: about 3 words are copied in per sample. 256^3, 256 views: TEX 13.7 ms,
-// HYBRID 8.4, STAGE 7.34, with the shared-memory reads at 88% of their rate; 512^3: TEX 218 ms,
-// HYBRID 133, STAGE 116. 16-bit volumes keep the packed texture (one gather a sample, 110 ms
-// at 512^3): staged in slice pairs they took the same time, bound by instruction issue.
+// What bounds the other layouts is the L1TEX unit: a texture gather returns 32 B a clock and
+// SM, so each of a TEX sample's two gathers (one for 16-bit slice pairs) takes it 16 clocks
+// per warp, whatever the cache hit rate. Shared memory returns 128 B a clock: an FP32
+// sample's eight 32-bit reads take 15.9 clocks per warp with their bank conflicts (the 32
+// lanes' texels lie in a patch of about 40 words, so two lanes of some bank usually differ).
+// Neighbouring rays share texels: about 3 words are copied in per sample. FP32, 256^3, 256
+// views: TEX 13.7 ms, HYBRID 8.4, STAGE 7.24, with the shared-memory reads at 88% of their
+// rate; 512^3: TEX 218 ms, HYBRID 133, STAGE 110. 16-bit volumes read four words of slice pairs
+// per sample and are bound by issue (60 instructions per sample at 85%), no faster than the
+// texture alone; together they are (RSG_SHARE16).
 //
 // A block is one detector tile of one view (256 rays) plus a producer warp. The rays march
 // across the planes of the axis (x or y) that the tile's central ray runs along. The volume
@@ -21,8 +22,9 @@
 // largest C whose C + 2 planes of the window fit a stage, and issues one
 // cp.async.bulk.tensor per plane (no multicast; this GPU's own buffer; texels off the volume
 // come back as the copy's zero fill, which is the reference's texture border). The window's
-// width W is one of a few values = 8 modulo 16 words: the four rows (z) of a warp's 8 u x 4 v
-// rays then fall on different eights of the 32 banks. The rays of a block stay within a
+// width W is one of a few values that put the four rows (z) of a warp's 8 u x 4 v rays on
+// different banks (256^3: {24, 40, 52, 68, 84} 7.25 ms, {24, 40, 56, 72, 88} 7.36,
+// {36, 44, 52, 68, 84} 7.75). The rays of a block stay within a
 // chunk of each other, so a plane is staged once per block.
 //
 // A ray's samples are the repeated additions and the arithmetic of rs_device.cuh whatever
@@ -47,15 +49,28 @@ constexpr int RSG_STAGES = 2;
 // 2 x 12288 8.25 ms, 3 x 8192 7.43, 4 x 6912 7.34, 5 x 5440 7.74, 6 x 4608 8.71: more blocks
 // hide the waits at chunk ends, shorter chunks stage their two shared planes more often).
 constexpr int RSG_CAP = 6912, RSG_MIN_BLOCKS = 4;
+// Sixteenths of the blocks that gather from the packed texture instead (16-bit volumes): the
+// gathers are bound by the texture's return path, staged samples by instruction issue, so
+// blocks of both kinds on an SM overlap. 384^3, 384 views, BF16: all gathered 34.7 ms, 12
+// sixteenths 31.6, 10 31.0, 8 31.3, none 34.6. FP32 volumes take none (2 sixteenths would gain
+// 1.5% for a texture beside the copies).
+constexpr int RSG_SHARE16 = 10;
 constexpr int RSG_CMAX = 30;            // planes of a chunk + 2 <= 32 lanes of the producer
 constexpr int RSG_WIDTHS = 5, RSG_HEIGHTS = 8;
-__host__ __device__ __forceinline__ int rsg_width(int i) { return 24 + 16 * i; }  // 24, 40, 56, 72, 88
+__host__ __device__ __forceinline__ int rsg_width(int i) { return i < 2 ? 24 + 16 * i : 20 + 16 * i; }  // 24, 40, 52, 68, 84
 __host__ __device__ __forceinline__ int rsg_height(int j) { return j < 5 ? 8 + 2 * j : j < 7 ? 4 * j : 32; }  // 8..16, 20, 24, 32
+
+// Slices of a copy: FP32 one word per voxel, slices 0 .. nz - 1; 16-bit storage one word per
+// slice pair (k, k + 1), low and high half, k = -1 .. nz - 1.
+template <typename Tv>
+__host__ __device__ __forceinline__ int rsg_slices(int nz) { return sizeof(Tv) == 4 ? nz : nz + 1; }
 
 struct RsStageSrc {              // what the kernel reads
     const CUtensorMap* maps;     // [axis: 0 = y-march, 1 = x-march][width][height]
-    const float* rows;           // the [z][y][x] copy
+    const unsigned* rows;        // the [z][y][x] copy
     int px;                      // its row pitch in words
+    unsigned long long tex;      // the packed texture (16-bit volumes)
+    int share;                   // sixteenths of the blocks that gather from it (RSG_SHARE16)
 };
 
 struct __align__(16) RsChunk {
@@ -90,34 +105,53 @@ __device__ __forceinline__ void rsg_init(RsStageShared* sh) {
     }
 }
 
-// One sample from the stage: a = the address of its texel (m, t, z), pp = bytes of a plane.
-template <int W, bool XM>
-__device__ __forceinline__ float rsg_sample(unsigned a, unsigned pp, const RsSample& s) {
+// The texels of a sample whose (m, t, z) is at address a, pp = bytes of a plane: the slices
+// lo and up in tld4 order, (i, j+1), (i+1, j+1), (i+1, j), (i, j).
+template <typename Tv, int W, bool XM>
+__device__ __forceinline__ void rsg_texels(unsigned a, unsigned pp, float4& lo, float4& up) {
     const unsigned b = a + pp;
-    float4 lo, up;  // tld4 order: (i, j+1), (i+1, j+1), (i+1, j), (i, j)
-    lo.w = lds_f32<0>(a);
-    up.w = lds_f32<W * 4>(a);
-    const float lt = lds_f32<4>(a), ut = lds_f32<W * 4 + 4>(a);
-    const float lm = lds_f32<0>(b), um = lds_f32<W * 4>(b);
-    lo.y = lds_f32<4>(b);
-    up.y = lds_f32<W * 4 + 4>(b);
-    lo.x = XM ? lt : lm;  // t is y for an x-march
-    lo.z = XM ? lm : lt;
-    up.x = XM ? ut : um;
-    up.z = XM ? um : ut;
-    return trilerp(lo, up, s);
+    if constexpr (sizeof(Tv) == 4) {
+        lo.w = lds_f32<0>(a);
+        up.w = lds_f32<W * 4>(a);
+        const float lt = lds_f32<4>(a), ut = lds_f32<W * 4 + 4>(a);
+        const float lm = lds_f32<0>(b), um = lds_f32<W * 4>(b);
+        lo.y = lds_f32<4>(b);
+        up.y = lds_f32<W * 4 + 4>(b);
+        lo.x = XM ? lt : lm;  // t is y for an x-march
+        lo.z = XM ? lm : lt;
+        up.x = XM ? ut : um;
+        up.z = XM ? um : ut;
+    } else {
+        auto word = [](float f) { return __float_as_uint(f); };
+        unpack_pair(word(lds_f32<0>(a)), lo.w, up.w, (Tv*)nullptr);
+        const unsigned wt = word(lds_f32<4>(a)), wm = word(lds_f32<0>(b));
+        unpack_pair(word(lds_f32<4>(b)), lo.y, up.y, (Tv*)nullptr);
+        unpack_pair(XM ? wt : wm, lo.x, up.x, (Tv*)nullptr);
+        unpack_pair(XM ? wm : wt, lo.z, up.z, (Tv*)nullptr);
+    }
 }
 
 // One sample from global memory (the [z][y][x] copy), zero outside the volume.
+template <typename Tv>
 __device__ __forceinline__ float rsg_global(const RsStageSrc& sv, int nx, int ny, int nz, const RsSample& s) {
     if (!rs_inside(s, (float)nx, (float)ny, (float)nz)) return 0.f;
     const int i = s.ix - FLOOR_KBITS, j = s.iy - FLOOR_KBITS, k = s.iz - FLOOR_KBITS;
-    auto texel = [&](int x, int y, int z) {
-        return x >= 0 && y >= 0 && z >= 0 && x < nx && y < ny && z < nz ? __ldg(sv.rows + ((long)z * ny + y) * sv.px + x)
-                                                                        : 0.f;
+    auto word = [&](int x, int y, int z) {
+        return x >= 0 && y >= 0 && z >= 0 && x < nx && y < ny && z < rsg_slices<Tv>(nz)
+                   ? __ldg(sv.rows + ((long)z * ny + y) * sv.px + x)
+                   : 0u;
     };
-    const float4 lo = make_float4(texel(i, j + 1, k), texel(i + 1, j + 1, k), texel(i + 1, j, k), texel(i, j, k));
-    const float4 up = make_float4(texel(i, j + 1, k + 1), texel(i + 1, j + 1, k + 1), texel(i + 1, j, k + 1), texel(i, j, k + 1));
+    float4 lo, up;
+    if constexpr (sizeof(Tv) == 4) {
+        auto texel = [&](int x, int y, int z) { return __uint_as_float(word(x, y, z)); };
+        lo = make_float4(texel(i, j + 1, k), texel(i + 1, j + 1, k), texel(i + 1, j, k), texel(i, j, k));
+        up = make_float4(texel(i, j + 1, k + 1), texel(i + 1, j + 1, k + 1), texel(i + 1, j, k + 1), texel(i, j, k + 1));
+    } else {
+        unpack_pair(word(i, j + 1, k + 1), lo.x, up.x, (Tv*)nullptr);
+        unpack_pair(word(i + 1, j + 1, k + 1), lo.y, up.y, (Tv*)nullptr);
+        unpack_pair(word(i + 1, j, k + 1), lo.z, up.z, (Tv*)nullptr);
+        unpack_pair(word(i, j, k + 1), lo.w, up.w, (Tv*)nullptr);
+    }
     return trilerp(lo, up, s);
 }
 
@@ -159,6 +193,7 @@ __device__ __forceinline__ void rsg_corners(const DevGeom& g, RsStageShared* sh,
 }
 
 // The producer warp: chunks from plane floor `lo` to `hi` (marching up) or from `hi` down.
+template <typename Tv>
 __device__ __forceinline__ void rsg_produce(const DevGeom& g, const RsStageSrc& sv, float* stages, RsStageShared* sh,
                                             unsigned& turn, bool xm, bool upward, float2 src, int lo, int hi,
                                             unsigned* err) {
@@ -182,7 +217,7 @@ __device__ __forceinline__ void rsg_produce(const DevGeom& g, const RsStageSrc& 
         const int t0 = sane ? (int)tl & ~3 : 0;  // the copy's rows start on 16 bytes
         const int z0 = sane ? (int)zl : 0;
         const int wn = sane ? (int)th + 2 - t0 : 1 << 20;
-        const int hn = sane ? (int)zh + 2 - z0 : 1 << 20;
+        const int hn = sane ? (int)zh + (sizeof(Tv) == 4 ? 2 : 1) - z0 : 1 << 20;
         int wi = 0, hj = 0;
         while (wi < RSG_WIDTHS && rsg_width(wi) < wn) ++wi;
         while (hj < RSG_HEIGHTS && rsg_height(hj) < hn) ++hj;
@@ -220,7 +255,8 @@ __device__ __forceinline__ void rsg_produce(const DevGeom& g, const RsStageSrc& 
         }
         __syncwarp();
         if (ok && lane < n + 2)
-            tma_load_3d(stages + s * RSG_CAP + lane * bpp, maps + bw * RSG_HEIGHTS + bh, bt, bz, plane0 + lane, &sh->full[s]);
+            tma_load_3d(stages + s * RSG_CAP + lane * bpp, maps + bw * RSG_HEIGHTS + bh, bt, bz + (sizeof(Tv) == 4 ? 0 : 1),
+                        plane0 + lane, &sh->full[s]);
         ++turn;
     }
     // the copies in flight land before the block may exit
@@ -230,7 +266,7 @@ __device__ __forceinline__ void rsg_produce(const DevGeom& g, const RsStageSrc& 
 
 // One tile of view p (as rs_tile; all RSG_THREADS threads call it). turn: the block's count
 // of chunks, carried from tile to tile.
-template <int MODE, typename To, int EPI, typename Tr = To>
+template <int MODE, typename Tv, typename To, int EPI, typename Tr = To>
 __device__ __forceinline__ void rs_stage_tile(const DevGeom& g, const RsStageSrc& sv, unsigned char* smem,
                                               unsigned& turn, const OutView<To>& out, const OutView<Tr>& real,
                                               double* __restrict__ norm, int p, int ut, int vt, unsigned* err) {
@@ -292,7 +328,7 @@ __device__ __forceinline__ void rs_stage_tile(const DevGeom& g, const RsStageSrc
     const int lo = sh->lo, hi = sh->hi;
     float acc = 0.f;
     if (warp >= 8) {
-        rsg_produce(g, sv, stages, sh, turn, xm, upward, src, lo, hi, err);
+        rsg_produce<Tv>(g, sv, stages, sh, turn, xm, upward, src, lo, hi, err);
     } else {
         const float dx = g.dx;
         const float2 SXY = make_float2(r.sx, r.sy);
@@ -307,7 +343,7 @@ __device__ __forceinline__ void rs_stage_tile(const DevGeom& g, const RsStageSrc
                 C = fadd(C, r.sz);
             }
         };
-        auto global = [&](const RsSample& sp) { return rsg_global(sv, g.nx, g.ny, g.nz, sp); };
+        auto global = [&](const RsSample& sp) { return rsg_global<Tv>(sv, g.nx, g.ny, g.nz, sp); };
         auto chunks = [&](auto axis) {
             constexpr bool XM = decltype(axis)::value;
             for (bool more = lo <= hi; more;) {
@@ -329,15 +365,17 @@ __device__ __forceinline__ void rs_stage_tile(const DevGeom& g, const RsStageSrc
                     march(cnt, [&](const RsSample& sp) {
                         const unsigned a = (unsigned)(XM ? sp.ix : sp.iy) * ch.pp +
                                            ((unsigned)sp.iz * (W * 4u) + ((unsigned)(XM ? sp.iy : sp.ix) * 4u + ch.bias));
-                        return rsg_sample<W, XM>(a, ch.pp, sp);
+                        float4 lo, up;
+                        rsg_texels<Tv, W, XM>(a, ch.pp, lo, up);
+                        return trilerp(lo, up, sp);
                     });
                 };
                 switch (ch.w_last & (RSG_LAST - 1)) {
                     case 24: staged(std::integral_constant<int, 24>{}); break;
                     case 40: staged(std::integral_constant<int, 40>{}); break;
-                    case 56: staged(std::integral_constant<int, 56>{}); break;
-                    case 72: staged(std::integral_constant<int, 72>{}); break;
-                    case 88: staged(std::integral_constant<int, 88>{}); break;
+                    case 52: staged(std::integral_constant<int, 52>{}); break;
+                    case 68: staged(std::integral_constant<int, 68>{}); break;
+                    case 84: staged(std::integral_constant<int, 84>{}); break;
                     default: march(cnt, global); break;
                 }
                 __syncwarp();

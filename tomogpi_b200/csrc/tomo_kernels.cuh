@@ -350,20 +350,24 @@ void rs_tex_destroy(RsTexture* t);
 // amax (optional, 16-bit textures filled by conversion): FP16 range guard scale source.
 cudaError_t rs_tex_fill(const void* vol, tomo_dtype vdt, int nx, int ny, int nz, const RsTexture& t, cudaStream_t st,
                         const unsigned* amax = nullptr);
-// STAGE resources (rs_stage.cuh): the FP32 volume's two copies and their tensor maps. What
-// TEX stands for with FP32 volumes wherever the geometry allows it.
+// STAGE resources (rs_stage.cuh): the volume's two copies in 32-bit words (FP32, or pairs of
+// 16-bit slices) and their tensor maps. What TEX stands for wherever the geometry allows it;
+// 16-bit volumes have the packed texture beside them, which part of the blocks gather from.
 struct RsStage {
     void *rows = nullptr, *cols = nullptr, *maps = nullptr;
+    tomo_dtype dt = TOMO_F32;
     int px = 0, py = 0;  // row pitches of the copies, in words
 };
-bool rs_stage_supported(const DevGeom& g);
-cudaError_t rs_stage_create(int nx, int ny, int nz, RsStage* t);
+bool rs_stage_supported(const DevGeom& g, tomo_dtype dt);
+cudaError_t rs_stage_create(int nx, int ny, int nz, tomo_dtype dt, RsStage* t);
 void rs_stage_destroy(RsStage* t);
-// Fills the copies from a dense device volume.
-cudaError_t rs_stage_fill(const float* vol, int nx, int ny, int nz, const RsStage& t, cudaStream_t st);
-// Grid as HYBRID's (rs_grid_blocks); bounded waits report ERR_TIMEOUT in *err.
-cudaError_t launch_rs_stage(int mode, int epi, const DevGeom& g, const RsStage& t, const OutView<void>& out,
-                            tomo_dtype odt, const OutView<void>& real, tomo_dtype rdt, double* norm, unsigned* err,
+// Fills the copies from a dense device volume (FP32, or of the copies' type).
+cudaError_t rs_stage_fill(const void* vol, tomo_dtype vdt, int nx, int ny, int nz, const RsStage& t, cudaStream_t st,
+                          const unsigned* amax = nullptr);
+size_t rs_stage_grid_blocks(const DevGeom& g);  // blocks of a launch (the EPI_NORM partials it writes)
+// Bounded waits report ERR_TIMEOUT in *err.
+cudaError_t launch_rs_stage(int mode, int epi, const DevGeom& g, const RsStage& t, unsigned long long tex,
+                            const OutView<void>& out, tomo_dtype odt, const OutView<void>& real, tomo_dtype rdt, double* norm, unsigned* err,
                             cudaStream_t st);
 void rs_tex_preload();
 int rs_tex_max_layers();
