@@ -420,7 +420,7 @@ def tuned(t, cfg, storage, dev):
     from tomogpi_b200 import autotune
 
     r = autotune.tune(cfg, storage, device=dev.index or 0)
-    return {"rs_layout": r["rs_layout"], "vi_zc": 1}
+    return {"rs_layout": r["batch_layout"], "vi_zc": 1}
 
 
 def single_job_fp32_ms(t, torch, dev, cfg, g, iters=2):
@@ -669,9 +669,11 @@ def run_ours(args):
     proj_avg = st["proj_ms"] / max(st["proj_launches"], 1)
     back_avg = st["back_ms"] / max(st["back_launches"], 1)
     if st["proj_ms"] >= st["back_ms"]:
-        kern, avg_ms, alg_bytes = "rs_project_kernel", proj_avg, 8 * 4 * samples + 4 * rays
+        # "tex" with an FP32 volume is staged in shared memory
+        kern = "rs_stage_kernel" if tuned_f32["rs_layout"] == "tex" else "rs_project_kernel"
+        avg_ms, alg_bytes = proj_avg, 8 * 4 * samples + 4 * rays
     else:
-        kern, avg_ms, alg_bytes = "vi_back_kernel", back_avg, 4 * 4 * U + 4 * nvox
+        kern, avg_ms, alg_bytes = "vi_back_tma_kernel", back_avg, 4 * 4 * U + 4 * nvox
     achieved = alg_bytes / (avg_ms / 1e3) / 1e9
     kkey = f"{kern}:{tuned_f32['rs_layout']}" if kern == "rs_project_kernel" else kern
     traffic = profiled_traffic(kkey)
@@ -691,8 +693,8 @@ def run_ours(args):
                 "dram_gbs": None if dram_gbs is None else round(dram_gbs, 1),
                 "dram_frac": None if dram_gbs is None else round(dram_gbs / peak, 4),
                 "limiter": limits,
-                "vi_limiter": profiled_limits("vi_back_tma_kernel" if tuned_f32.get("vi_layout") == "tma"
-                                              else "vi_back_kernel"),
+                "vi_limiter": profiled_limits("vi_back_tma_kernel" if tuned_f32["vi_zc"] == 1
+                                              or tuned_f32.get("vi_layout") == "tma" else "vi_back_kernel"),
                 "traffic": traffic, "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": round(avg_ms, 3),
                 "rs_avg_launch_ms": round(proj_avg, 3), "vi_avg_launch_ms": round(back_avg, 3),
                 "rs_samples_per_launch": samples,

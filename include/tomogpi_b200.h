@@ -119,7 +119,9 @@ tomo_status tomo_context_geometry(const tomo_context* ctx, float* scalars, float
    0 = zero-bordered padded copy (1x), 1 = 2x2x2 texel cells (8x the volume's bytes, one
    aligned 32 B / 16 B vector load per sample), 2 = 2D layered texture in the storage type
    (FP32, or the raw bits of BF16 / FP16), one layer per z slice, read with 4-texel gathers
-   (depths beyond the device's layer limit use 1), 3 = the texture for the lower slice of
+   (depths beyond the device's layer limit use 1) -- or, where a detector tile's windows of
+   the volume fit, staged in shared memory by TMA from two copies of it (8 B a voxel; FP32 in
+   place of the texture, 16-bit volumes from 128^3 on beside it), the same results --, 3 = the texture for the lower slice of
    each sample plus, for the upper slice, the slice's four footprint texels stored together
    (FP32 only; 8x the volume's bytes besides the texture), 4 = faces across the axis the
    view's rays mostly run along, even faces in a layered texture and odd faces as stored
@@ -129,11 +131,11 @@ tomo_status tomo_context_geometry(const tomo_context* ctx, float* scalars, float
    launch shape: rays of one warp along u (8, 16 or 32, the rest of its 32 along v; 0 = 8)
    and of one 256-thread block along u (16, 32, 64 or 128, at least rs_warp_u; 0 = 32).
    vi_layout: sinogram read by the VI
-   backprojectors, 0 = zero-bordered padded copy (four scalar loads per voxel and view),
+   backprojectors, 0 = with 16 slices per thread as 2 (any type and width, through an FP32
+   copy where needed), else a zero-bordered padded copy (four scalar loads per voxel and view),
    1 = 2D layered texture, one layer per view, one 4-texel gather per voxel and view (view
    counts beyond the layer limit use 0), 2 = FP32 sinogram windows staged in shared memory
-   by TMA, one per (voxel tile, view), read by the bilinear samples (FP32 sinograms with nu
-   a multiple of 4; otherwise 0). Set before creating solvers on the context. */
+   by TMA, one per (voxel tile, view), read by the bilinear samples. Set before creating solvers on the context. */
 typedef struct {
     int32_t rs_layout;
     int32_t vi_zc;       /* VI: 16-slice chunks per thread (1, 2 or 4; 0 = default 1) */

@@ -1,9 +1,11 @@
 """Autotuner: per size class, pick the RS input layout and the VI form by timing the
 candidates on the device, and cache the choice.
 
-Candidates: RS layout in {tex, hybrid, cell8, plain}; VI slices per thread in
-{16, 32, 64} (vi_zc 1, 2, 4) from the padded sinogram, or 16 slices from sinogram windows
-staged in shared memory by TMA (vi_layout "tma"). The trials run the first k and 2k views of the job's own
+Candidates: RS layout in {tex, hybrid, cell8, plain, march}; VI slices per thread in
+{16, 32, 64} (vi_zc 1, 2, 4; 16 staged in shared memory by TMA, the others from the padded
+sinogram), and the staged form by name (vi_layout "tma"). "tex" is staged too where the
+geometry allows it; the batch's queue gathers from the texture, so its layout is picked with a
+trial of that form ("batch_layout"). The trials run the first k and 2k views of the job's own
 geometry, with CUDA-event timing after a warm-up, and are extrapolated to the job's view
 count. Results are cached in JSON (``$TOMOGPI_B200_TUNE_CACHE`` or
 ``~/.cache/tomogpi_b200/autotune.json``) keyed by the GPU name and the size class.
@@ -93,7 +95,7 @@ def extrapolate(t_k: float, t_2k: float, k: int, views: int) -> float:
 
 def tune(cfg: ConfigCT, storage: str = "f32", device: int = 0, trial_views: int = 64, vi_zcs=(1, 2, 4),
          force: bool = False) -> dict:
-    """Returns {"rs_layout", "vi_zc", "trials", "trial_views"} for this size class. Each
+    """Returns {"rs_layout", "vi_zc", "vi_layout", "batch_layout", "trials", "trial_views"} for this size class. Each
     candidate runs over the first k and 2k views of the job's geometry; `trials` holds the
     times extrapolated to the job's view count (the fixed per-call cost -- e.g. filling a
     layout's input buffers -- would otherwise dominate a short trial)."""
@@ -124,6 +126,10 @@ def tune(cfg: ConfigCT, storage: str = "f32", device: int = 0, trial_views: int 
             for lay in layouts:
                 ctx.set_tuning(rs_layout=lay)
                 raw[(f"rs_{lay}", views)] = _time(lambda: ctx.project("RS", vol, out=sino), reps=2)
+            # 128 rays wide, a block's windows fit no stage: the texture's gathers
+            ctx.set_tuning(rs_layout="tex", rs_tile_u=128)
+            raw[("gather", views)] = _time(lambda: ctx.project("RS", vol, out=sino), reps=2)
+            ctx.set_tuning(rs_tile_u=32)
             res = torch.rand(sub.sinogram_shape, device=dev)
             dj = torch.empty(sub.volume_shape, device=dev)
             for zc in vi_zcs:
@@ -137,7 +143,9 @@ def tune(cfg: ConfigCT, storage: str = "f32", device: int = 0, trial_views: int 
     trials = {}
     for name in {n for n, _ in raw}:
         trials[name] = extrapolate(raw[(name, k)], raw[(name, k2)], k, P) if k2 > k else raw[(name, k)]
-    out = dict(pick(trials), trials=trials, trial_views=[k, k2])
+    gather = trials.pop("gather")
+    queue = {"tex": gather, **{k[3:]: v for k, v in trials.items() if k in ("rs_cell8", "rs_plain")}}
+    out = dict(pick(trials), batch_layout=min(queue, key=queue.get), trials=trials, trial_views=[k, k2])
     cache[key] = out
     _save()
     return out

@@ -315,11 +315,10 @@ tomo_status tomo_context_create_views(const tomo_config_ct* cfg, int device, int
     TOMO_CHECK_ARG(device >= 0 && device < ndev, "tomo_context_create: no such CUDA device");
     tomo_context* ctx = new tomo_context();
     ctx->device = device;
-    // Measured on B200 (512^3, 512 views). RS: texture gathers 218 ms (FP32) / 156 ms (BF16),
-    // 2x2x2 cells 269 / 155 ms, padded scalar loads 367 ms; at 1024^3 BF16 the texture wins
-    // 2.49 s to 5.25 s (the cells' 8x footprint overflows L2). VI: 16 slices per thread 80 ms,
-    // 32 slices 95 ms (64 registers halve residency), 64 slices 180 ms; the texture form of
-    // the sinogram 111 ms.
+    // Measured on B200 (512^3, 512 views). RS, FP32: staged 109 ms (what TEX runs), hybrid 133,
+    // texture gathers 218, 2x2x2 cells 269, padded scalar loads 367; BF16: staged and gathered
+    // 97, gathered 110, cells 155. VI: staged, 16 slices per thread 43.4 ms; padded 72, with 32
+    // slices 79; the texture form of the sinogram 111.
     ctx->tuning.rs_layout = RS_LAYOUT_TEX;
     ctx->tuning.vi_zc = 1;
     ctx->tuning.vi_layout = 0;

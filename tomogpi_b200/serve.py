@@ -209,7 +209,7 @@ class Server:
         if self.tuner is None:
             return {"rs_layout": "tex", "vi_zc": 1}
         t = self.tuner(cfg, self.params.storage)
-        return {"rs_layout": t["rs_layout"], "vi_zc": min(int(t["vi_zc"]), 2)}  # the batch runs zc 1 or 2
+        return {"rs_layout": t.get("batch_layout", t["rs_layout"]), "vi_zc": min(int(t["vi_zc"]), 2)}  # the batch runs zc 1 or 2
 
     def submit(self, req: Request) -> None:
         if req.tuning is None:
