@@ -5,11 +5,11 @@
 // What bounds the other layouts is the L1TEX unit: a texture gather returns 32 B a clock and
 // SM, so each of a TEX sample's two gathers (one for 16-bit slice pairs) takes it 16 clocks
 // per warp, whatever the cache hit rate. Shared memory returns 128 B a clock: an FP32
-// sample's eight 32-bit reads take 15.9 clocks per warp with their bank conflicts (the 32
+// sample's eight 32-bit reads take 14.7 clocks per warp with their bank conflicts (the 32
 // lanes' texels lie in a patch of about 40 words, so two lanes of some bank usually differ).
 // Neighbouring rays share texels: about 3 words are copied in per sample. FP32, 256^3, 256
-// views: TEX 13.7 ms, HYBRID 8.4, STAGE 7.24, with the shared-memory reads at 88% of their
-// rate; 512^3: TEX 218 ms, HYBRID 133, STAGE 110. 16-bit volumes read four words of slice pairs
+// views: TEX 13.7 ms, HYBRID 8.4, STAGE 7.16, with the shared-memory reads at 87% of their
+// rate; 512^3: TEX 218 ms, HYBRID 133, STAGE 109. 16-bit volumes read four words of slice pairs
 // per sample and are bound by issue (60 instructions per sample at 85%), no faster than the
 // texture alone; together they are (RSG_SHARE16).
 //
