@@ -115,3 +115,17 @@ def test_staged_backprojection_equals_padded(tomo, spec, dtype):
                 assert torch.equal(v, ref), k
         torch.cuda.synchronize()
         assert ctx.errors() == 0
+
+
+def test_staged_copies_remade_at_the_same_address(tomo):
+    """Copies of another type or size, made where earlier ones were freed: each projection is read
+    through its own tensor maps (the type of one context's volume alternates; contexts of other
+    sizes follow one another)."""
+    for n, views in ((128, 45), (131, 45), (128, 44)):
+        cfg = _cfg(tomo, n, n, n, n, n, views, 2.0)
+        vol = torch.rand(cfg.volume_shape, device="cuda")
+        with tomo.Context(cfg) as ctx, tomo.Context(cfg) as plain:
+            plain.set_tuning(rs_layout="cell8")
+            for dt in (torch.float32, torch.bfloat16, torch.float32, torch.float16, torch.bfloat16):
+                v = vol.to(dt)
+                assert torch.equal(ctx.project("RS", v, dtype=torch.float32), plain.project("RS", v, dtype=torch.float32)), (n, dt)

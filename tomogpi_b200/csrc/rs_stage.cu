@@ -2,7 +2,7 @@
 // kernel, the two volume copies that it reads and their tensor maps.
 #include <algorithm>
 #include <atomic>
-#include <vector>
+#include <new>
 
 #include "rs_stage.cuh"
 
@@ -10,7 +10,8 @@ namespace tomo {
 
 template <int MODE, typename Tv, typename To, int EPI, typename Tr>
 __global__ void __launch_bounds__(RSG_THREADS, RSG_MIN_BLOCKS)
-    rs_stage_kernel(DevGeom g, RsStageSrc sv, OutView<To> out, OutView<Tr> real, double* __restrict__ norm, unsigned* err) {
+    rs_stage_kernel(DevGeom g, const __grid_constant__ RsStageMaps maps, RsStageSrc sv, OutView<To> out, OutView<Tr> real,
+                    double* __restrict__ norm, unsigned* err) {
     extern __shared__ __align__(1024) unsigned char smem[];
     // blockIdx.z: the v-tiles of the views whose rays run along x, then those of the others, so
     // that the resident blocks read one of the two copies
@@ -28,7 +29,7 @@ __global__ void __launch_bounds__(RSG_THREADS, RSG_MIN_BLOCKS)
     }
     rsg_init(reinterpret_cast<RsStageShared*>(smem));
     unsigned turn = 0;
-    rs_stage_tile<MODE, Tv, To, EPI, Tr>(g, sv, smem, turn, out, real, norm, p, blockIdx.y, vt, err);
+    rs_stage_tile<MODE, Tv, To, EPI, Tr>(g, maps, sv, smem, turn, out, real, norm, p, blockIdx.y, vt, err);
 }
 
 // The two copies of a volume [z][y][x] of type Ti: a block reads a 32 x 32 tile of a slice
@@ -87,19 +88,18 @@ cudaError_t rs_stage_create(int nx, int ny, int nz, tomo_dtype dt, RsStage* t) {
     *t = RsStage();
     const int nzr = stage_slices(dt, nz);
     const int px = pitch4(nx), py = pitch4(ny);
-    // one allocation: rows, then cols, then the maps, each from a 256-byte boundary
-    auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
-    const size_t rb = up((size_t)nzr * ny * px * 4), cb = up((size_t)nzr * nx * py * 4);
+    // one allocation: rows, then cols from a 256-byte boundary
+    const size_t rb = ((size_t)nzr * ny * px * 4 + 255) & ~(size_t)255, cb = (size_t)nzr * nx * py * 4;
     char* base = nullptr;
-    cudaError_t e = cudaMalloc((void**)&base, rb + cb + 2 * RSG_WIDTHS * RSG_HEIGHTS * sizeof(CUtensorMap));
+    cudaError_t e = cudaMalloc((void**)&base, rb + cb);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return e;
     }
     t->rows = base;
     t->cols = base + rb;
-    t->maps = base + rb + cb;
-    std::vector<CUtensorMap> m(2 * RSG_WIDTHS * RSG_HEIGHTS);
+    t->maps = new (std::nothrow) RsStageMaps;
+    if (!t->maps) e = cudaErrorMemoryAllocation;
     for (int o = 0; o < 2 && e == cudaSuccess; ++o) {
         // dimensions (t, z, m): rows [z][y][x] march along y, cols [z][x][y] along x
         void* p = o ? t->cols : t->rows;
@@ -110,14 +110,12 @@ cudaError_t rs_stage_create(int nx, int ny, int nz, tomo_dtype dt, RsStage* t) {
         for (int i = 0; i < RSG_WIDTHS && e == cudaSuccess; ++i)
             for (int j = 0; j < RSG_HEIGHTS && e == cudaSuccess; ++j) {
                 const cuuint32_t box[3] = {(cuuint32_t)rsg_width(i), (cuuint32_t)rsg_height(j), 1};
-                if (tma_encode_fn()(&m[(o * RSG_WIDTHS + i) * RSG_HEIGHTS + j], CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, p, dims,
+                if (tma_encode_fn()(&t->maps->m[o][i][j], CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, p, dims,
                                     strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                                     CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
                     e = cudaErrorInvalidValue;
             }
     }
-    if (e == cudaSuccess)
-        e = cudaMemcpy(t->maps, m.data(), m.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         rs_stage_destroy(t);
         cudaGetLastError();
@@ -131,6 +129,7 @@ cudaError_t rs_stage_create(int nx, int ny, int nz, tomo_dtype dt, RsStage* t) {
 
 void rs_stage_destroy(RsStage* t) {
     cudaFree(t->rows);  // the one allocation
+    delete t->maps;
     *t = RsStage();
 }
 
@@ -173,8 +172,8 @@ static cudaError_t launch_stage_k(const DevGeom& g, const RsStage& t, unsigned l
         if (e == cudaSuccess && dev < 64) ready.fetch_or(1ull << dev);
     }
     if (e != cudaSuccess) return e;
-    const RsStageSrc sv{(const CUtensorMap*)t.maps, (const unsigned*)t.rows, t.px, tex, sizeof(Tv) == 4 ? 0 : RSG_SHARE16};
-    k<<<stage_grid(g), RSG_THREADS, RSG_SMEM, st>>>(g, sv, out.as<To>(), real.as<Tr>(), norm, err);
+    const RsStageSrc sv{(const unsigned*)t.rows, t.px, tex, sizeof(Tv) == 4 ? 0 : RSG_SHARE16};
+    k<<<stage_grid(g), RSG_THREADS, RSG_SMEM, st>>>(g, *t.maps, sv, out.as<To>(), real.as<Tr>(), norm, err);
     return cudaGetLastError();
 }
 

@@ -65,8 +65,13 @@ __host__ __device__ __forceinline__ int rsg_height(int j) { return j < 5 ? 8 + 2
 template <typename Tv>
 __host__ __device__ __forceinline__ int rsg_slices(int nz) { return sizeof(Tv) == 4 ? nz : nz + 1; }
 
-struct RsStageSrc {              // what the kernel reads
-    const CUtensorMap* maps;     // [axis: 0 = y-march, 1 = x-march][width][height]
+// The copies' tensor maps, a kernel parameter (10 KB): maps in device memory would need a
+// proxy fence per block, since a freed copy's maps may have been at the same address.
+struct RsStageMaps {
+    CUtensorMap m[2][RSG_WIDTHS][RSG_HEIGHTS];  // [axis: 0 = y-march, 1 = x-march]
+};
+
+struct RsStageSrc {              // what the kernel reads beside them
     const unsigned* rows;        // the [z][y][x] copy
     int px;                      // its row pitch in words
     unsigned long long tex;      // the packed texture (16-bit volumes)
@@ -194,13 +199,12 @@ __device__ __forceinline__ void rsg_corners(const DevGeom& g, RsStageShared* sh,
 
 // The producer warp: chunks from plane floor `lo` to `hi` (marching up) or from `hi` down.
 template <typename Tv>
-__device__ __forceinline__ void rsg_produce(const DevGeom& g, const RsStageSrc& sv, float* stages, RsStageShared* sh,
+__device__ __forceinline__ void rsg_produce(const DevGeom& g, const RsStageMaps& maps, float* stages, RsStageShared* sh,
                                             unsigned& turn, bool xm, bool upward, float2 src, int lo, int hi,
                                             unsigned* err) {
     const int lane = threadIdx.x & 31;
     const float st0 = sh->st[0], st1 = sh->st[1], sz0 = sh->sz[0], sz1 = sh->sz[1], pad = rsg_pad(g);
     const bool along = sh->along;
-    const CUtensorMap* maps = sv.maps + (xm ? RSG_WIDTHS * RSG_HEIGHTS : 0);
     int cur = upward ? lo : hi;
     const unsigned first = turn;
     while (upward ? cur <= hi : cur >= lo) {
@@ -255,7 +259,7 @@ __device__ __forceinline__ void rsg_produce(const DevGeom& g, const RsStageSrc& 
         }
         __syncwarp();
         if (ok && lane < n + 2)
-            tma_load_3d(stages + s * RSG_CAP + lane * bpp, maps + bw * RSG_HEIGHTS + bh, bt, bz + (sizeof(Tv) == 4 ? 0 : 1),
+            tma_load_3d(stages + s * RSG_CAP + lane * bpp, &maps.m[xm][bw][bh], bt, bz + (sizeof(Tv) == 4 ? 0 : 1),
                         plane0 + lane, &sh->full[s]);
         ++turn;
     }
@@ -267,8 +271,8 @@ __device__ __forceinline__ void rsg_produce(const DevGeom& g, const RsStageSrc& 
 // One tile of view p (as rs_tile; all RSG_THREADS threads call it). turn: the block's count
 // of chunks, carried from tile to tile.
 template <int MODE, typename Tv, typename To, int EPI, typename Tr = To>
-__device__ __forceinline__ void rs_stage_tile(const DevGeom& g, const RsStageSrc& sv, unsigned char* smem,
-                                              unsigned& turn, const OutView<To>& out, const OutView<Tr>& real,
+__device__ __forceinline__ void rs_stage_tile(const DevGeom& g, const RsStageMaps& maps, const RsStageSrc& sv,
+                                              unsigned char* smem, unsigned& turn, const OutView<To>& out, const OutView<Tr>& real,
                                               double* __restrict__ norm, int p, int ut, int vt, unsigned* err) {
     RsStageShared* sh = reinterpret_cast<RsStageShared*>(smem);
     float* stages = reinterpret_cast<float*>(smem + RSG_HEADER);
@@ -328,7 +332,7 @@ __device__ __forceinline__ void rs_stage_tile(const DevGeom& g, const RsStageSrc
     const int lo = sh->lo, hi = sh->hi;
     float acc = 0.f;
     if (warp >= 8) {
-        rsg_produce<Tv>(g, sv, stages, sh, turn, xm, upward, src, lo, hi, err);
+        rsg_produce<Tv>(g, maps, stages, sh, turn, xm, upward, src, lo, hi, err);
     } else {
         const float dx = g.dx;
         const float2 SXY = make_float2(r.sx, r.sy);

@@ -353,8 +353,10 @@ cudaError_t rs_tex_fill(const void* vol, tomo_dtype vdt, int nx, int ny, int nz,
 // STAGE resources (rs_stage.cuh): the volume's two copies in 32-bit words (FP32, or pairs of
 // 16-bit slices) and their tensor maps. What TEX stands for wherever the geometry allows it;
 // 16-bit volumes have the packed texture beside them, which part of the blocks gather from.
+struct RsStageMaps;
 struct RsStage {
-    void *rows = nullptr, *cols = nullptr, *maps = nullptr;
+    void *rows = nullptr, *cols = nullptr;
+    RsStageMaps* maps = nullptr;  // host memory: a launch takes them by value
     tomo_dtype dt = TOMO_F32;
     int px = 0, py = 0;  // row pitches of the copies, in words
 };
