@@ -129,3 +129,19 @@ def test_staged_copies_remade_at_the_same_address(tomo):
             for dt in (torch.float32, torch.bfloat16, torch.float32, torch.float16, torch.bfloat16):
                 v = vol.to(dt)
                 assert torch.equal(ctx.project("RS", v, dtype=torch.float32), plain.project("RS", v, dtype=torch.float32)), (n, dt)
+
+
+@pytest.mark.parametrize("dtype,n,views", [(torch.float32, 128, 8), (torch.bfloat16, 128, 45)])
+def test_closed_contexts_give_their_copies_back(tomo, dtype, n, views):
+    """A closed context leaves no device memory behind: its two volume copies are 16 MiB (FP32)
+    at 128^3, so a leak of them shows after the second of six contexts."""
+    cfg = _cfg(tomo, n, n, n, n, n, views, 2.0)
+    vol = torch.rand(cfg.volume_shape, device="cuda").to(dtype)
+    out = torch.empty(cfg.sinogram_shape, device="cuda", dtype=dtype)
+    free = []
+    for _ in range(6):
+        with tomo.Context(cfg) as ctx:
+            ctx.project("RS", vol, out=out)
+            torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] - free[-1] < 8 << 20, free

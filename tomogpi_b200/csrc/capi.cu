@@ -368,6 +368,7 @@ tomo_status tomo_context_destroy(tomo_context* ctx) {
     cudaFree(ctx->rows);
     cudaFree(ctx->adj_scratch);
     rs_tex_destroy(&ctx->tex);
+    rs_stage_destroy(&ctx->stage);
     rs_tex_destroy(&ctx->vtex);
     cudaFree(ctx->d_ramp);
     cudaFree(ctx->h_vol);
