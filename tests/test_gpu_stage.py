@@ -145,3 +145,26 @@ def test_closed_contexts_give_their_copies_back(tomo, dtype, n, views):
             torch.cuda.synchronize()
         free.append(torch.cuda.mem_get_info()[0])
     assert free[0] - free[-1] < 8 << 20, free
+
+
+@pytest.mark.parametrize("dtype,n,views", [(torch.float32, 16, 4), (torch.bfloat16, 128, 40)])
+def test_staged_projection_bounded_wait_reports_timeout(tomo, dtype, n, views):
+    """With the test stall the producer issues no copy and the consumers' waits run out after
+    their one-second bound: the call returns, ERR_TIMEOUT (bit 1) is in the context's error word,
+    and the next call on the context is exact. A detector of one tile keeps it to a few blocks a
+    view (16-bit volumes: the ones that do not gather)."""
+    from tomogpi_b200 import _lib as L
+
+    cfg = _cfg(tomo, n, n, n, 128 if n == 128 else 16, 128 if n == 128 else 8, views, 2.0)
+    vol = torch.rand(cfg.volume_shape, device="cuda").to(dtype)
+    with tomo.Context(cfg, views=(0, 1) if n == 16 else None) as ctx:
+        ref = ctx.project("RS", vol)
+        torch.cuda.synchronize()
+        assert ctx.errors(clear=True) == 0
+        L.call("tomo_context_test_stall", ctx.handle, 1)
+        ctx.project("RS", vol)
+        torch.cuda.synchronize()
+        assert ctx.errors(clear=True) & 2
+        L.call("tomo_context_test_stall", ctx.handle, 0)
+        assert torch.equal(ctx.project("RS", vol), ref)
+        assert ctx.errors() == 0

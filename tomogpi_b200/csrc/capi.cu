@@ -266,7 +266,7 @@ tomo_status project_into(tomo_context* ctx, tomo_projector kind, const void* vol
             const tomo_status s = check_launch(rs_stage_fill(vol, vdt, g.nx, g.ny, g.nz, ctx->stage, st), "rs stage fill");
             if (s != TOMO_OK) return s;
             return check_launch(launch_rs_stage(kind == TOMO_PROJ_RS ? 0 : 1, epi, g, ctx->stage, ctx->tex.tex, out, odt, real,
-                                                TOMO_F32, norm, ctx->d_err, st),
+                                                TOMO_F32, norm, ctx->d_err, st, ctx->test_stall),
                                 "rs_stage_kernel");
         }
         if (layout != RS_LAYOUT_TEX &&  // HYBRID: the texture above plus its cell buffer

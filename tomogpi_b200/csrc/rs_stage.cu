@@ -11,7 +11,7 @@ namespace tomo {
 template <int MODE, typename Tv, typename To, int EPI, typename Tr>
 __global__ void __launch_bounds__(RSG_THREADS, RSG_MIN_BLOCKS)
     rs_stage_kernel(DevGeom g, const __grid_constant__ RsStageMaps maps, RsStageSrc sv, OutView<To> out, OutView<Tr> real,
-                    double* __restrict__ norm, unsigned* err) {
+                    double* __restrict__ norm, unsigned* err, int stall) {
     extern __shared__ __align__(1024) unsigned char smem[];
     // blockIdx.z: the v-tiles of the views whose rays run along x, then those of the others, so
     // that the resident blocks read one of the two copies
@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(RSG_THREADS, RSG_MIN_BLOCKS)
     }
     rsg_init(reinterpret_cast<RsStageShared*>(smem));
     unsigned turn = 0;
-    rs_stage_tile<MODE, Tv, To, EPI, Tr>(g, maps, sv, smem, turn, out, real, norm, p, blockIdx.y, vt, err);
+    rs_stage_tile<MODE, Tv, To, EPI, Tr>(g, maps, sv, smem, turn, out, real, norm, p, blockIdx.y, vt, err, stall);
 }
 
 // The two copies of a volume [z][y][x] of type Ti: a block reads a 32 x 32 tile of a slice
@@ -162,7 +162,7 @@ size_t rs_stage_grid_blocks(const DevGeom& g) {
 
 template <int MODE, int EPI, typename Tv, typename To, typename Tr>
 static cudaError_t launch_stage_k(const DevGeom& g, const RsStage& t, unsigned long long tex, const OutView<void>& out, const OutView<void>& real,
-                                  double* norm, unsigned* err, cudaStream_t st) {
+                                  double* norm, unsigned* err, cudaStream_t st, int stall) {
     auto k = rs_stage_kernel<MODE, Tv, To, EPI, Tr>;
     static std::atomic<unsigned long long> ready{0};  // devices on which the kernel may use its shared memory
     int dev = 0;
@@ -173,38 +173,38 @@ static cudaError_t launch_stage_k(const DevGeom& g, const RsStage& t, unsigned l
     }
     if (e != cudaSuccess) return e;
     const RsStageSrc sv{(const unsigned*)t.rows, t.px, tex, sizeof(Tv) == 4 ? 0 : RSG_SHARE16};
-    k<<<stage_grid(g), RSG_THREADS, RSG_SMEM, st>>>(g, *t.maps, sv, out.as<To>(), real.as<Tr>(), norm, err);
+    k<<<stage_grid(g), RSG_THREADS, RSG_SMEM, st>>>(g, *t.maps, sv, out.as<To>(), real.as<Tr>(), norm, err, stall);
     return cudaGetLastError();
 }
 
 template <int MODE, typename Tv>
 static cudaError_t launch_stage_e(int epi, const DevGeom& g, const RsStage& t, unsigned long long tex, const OutView<void>& out, tomo_dtype odt,
-                                  const OutView<void>& real, tomo_dtype rdt, double* norm, unsigned* err, cudaStream_t st) {
+                                  const OutView<void>& real, tomo_dtype rdt, double* norm, unsigned* err, cudaStream_t st, int stall) {
     using B = __nv_bfloat16;
     if (epi == EPI_STORE) {
         switch (odt) {
-            case TOMO_F32: return launch_stage_k<MODE, EPI_STORE, Tv, float, float>(g, t, tex, out, real, norm, err, st);
-            case TOMO_BF16: return launch_stage_k<MODE, EPI_STORE, Tv, B, B>(g, t, tex, out, real, norm, err, st);
-            case TOMO_F16: return launch_stage_k<MODE, EPI_STORE, Tv, __half, __half>(g, t, tex, out, real, norm, err, st);
+            case TOMO_F32: return launch_stage_k<MODE, EPI_STORE, Tv, float, float>(g, t, tex, out, real, norm, err, st, stall);
+            case TOMO_BF16: return launch_stage_k<MODE, EPI_STORE, Tv, B, B>(g, t, tex, out, real, norm, err, st, stall);
+            case TOMO_F16: return launch_stage_k<MODE, EPI_STORE, Tv, __half, __half>(g, t, tex, out, real, norm, err, st, stall);
         }
     } else if (epi == EPI_RESIDUAL) {
         switch (rdt) {
-            case TOMO_F32: return launch_stage_k<MODE, EPI_RESIDUAL, Tv, float, float>(g, t, tex, out, real, norm, err, st);
-            case TOMO_BF16: return launch_stage_k<MODE, EPI_RESIDUAL, Tv, float, B>(g, t, tex, out, real, norm, err, st);
-            case TOMO_F16: return launch_stage_k<MODE, EPI_RESIDUAL, Tv, float, __half>(g, t, tex, out, real, norm, err, st);
+            case TOMO_F32: return launch_stage_k<MODE, EPI_RESIDUAL, Tv, float, float>(g, t, tex, out, real, norm, err, st, stall);
+            case TOMO_BF16: return launch_stage_k<MODE, EPI_RESIDUAL, Tv, float, B>(g, t, tex, out, real, norm, err, st, stall);
+            case TOMO_F16: return launch_stage_k<MODE, EPI_RESIDUAL, Tv, float, __half>(g, t, tex, out, real, norm, err, st, stall);
         }
     } else if (epi == EPI_NORM) {
-        return launch_stage_k<MODE, EPI_NORM, Tv, float, float>(g, t, tex, out, real, norm, err, st);
+        return launch_stage_k<MODE, EPI_NORM, Tv, float, float>(g, t, tex, out, real, norm, err, st, stall);
     }
     return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_rs_stage(int mode, int epi, const DevGeom& g, const RsStage& t, unsigned long long tex, const OutView<void>& out,
                             tomo_dtype odt, const OutView<void>& real, tomo_dtype rdt, double* norm, unsigned* err,
-                            cudaStream_t st) {
+                            cudaStream_t st, int stall) {
 #define TOMO_STAGE(TV)                                                                          \
-    return mode == 0 ? launch_stage_e<0, TV>(epi, g, t, tex, out, odt, real, rdt, norm, err, st)     \
-                     : launch_stage_e<1, TV>(epi, g, t, tex, out, odt, real, rdt, norm, err, st);
+    return mode == 0 ? launch_stage_e<0, TV>(epi, g, t, tex, out, odt, real, rdt, norm, err, st, stall)     \
+                     : launch_stage_e<1, TV>(epi, g, t, tex, out, odt, real, rdt, norm, err, st, stall);
     switch (t.dt) {
         case TOMO_F32: TOMO_STAGE(float)
         case TOMO_BF16: TOMO_STAGE(__nv_bfloat16)

@@ -201,7 +201,8 @@ __device__ __forceinline__ void rsg_corners(const DevGeom& g, RsStageShared* sh,
 template <typename Tv>
 __device__ __forceinline__ void rsg_produce(const DevGeom& g, const RsStageMaps& maps, float* stages, RsStageShared* sh,
                                             unsigned& turn, bool xm, bool upward, float2 src, int lo, int hi,
-                                            unsigned* err) {
+                                            unsigned* err, int stall) {
+    if (stall) return;  // tests only: no copy, so every consumer wait runs out
     const int lane = threadIdx.x & 31;
     const float st0 = sh->st[0], st1 = sh->st[1], sz0 = sh->sz[0], sz1 = sh->sz[1], pad = rsg_pad(g);
     const bool along = sh->along;
@@ -230,7 +231,7 @@ __device__ __forceinline__ void rsg_produce(const DevGeom& g, const RsStageMaps&
         const unsigned ok = __ballot_sync(0xffffffffu, fits);
         const int s = turn % RSG_STAGES;
         const unsigned k = turn / RSG_STAGES;
-        if (k > 0 && !mbar_wait(&sh->empty[s], (k - 1) & 1)) {
+        if (k > 0 && !mbar_wait_warp(&sh->empty[s], (k - 1) & 1)) {
             if (lane == 0) {
                 atomicOr(err, ERR_TIMEOUT);
                 sh->abort_flag = 1;
@@ -265,7 +266,7 @@ __device__ __forceinline__ void rsg_produce(const DevGeom& g, const RsStageMaps&
     }
     // the copies in flight land before the block may exit
     for (unsigned q = turn - first < RSG_STAGES ? first : turn - RSG_STAGES; q != turn; ++q)
-        if (!mbar_wait(&sh->full[q % RSG_STAGES], (q / RSG_STAGES) & 1) && lane == 0) atomicOr(err, ERR_TIMEOUT);
+        if (!mbar_wait_warp(&sh->full[q % RSG_STAGES], (q / RSG_STAGES) & 1) && lane == 0) atomicOr(err, ERR_TIMEOUT);
 }
 
 // One tile of view p (as rs_tile; all RSG_THREADS threads call it). turn: the block's count
@@ -273,7 +274,7 @@ __device__ __forceinline__ void rsg_produce(const DevGeom& g, const RsStageMaps&
 template <int MODE, typename Tv, typename To, int EPI, typename Tr = To>
 __device__ __forceinline__ void rs_stage_tile(const DevGeom& g, const RsStageMaps& maps, const RsStageSrc& sv,
                                               unsigned char* smem, unsigned& turn, const OutView<To>& out, const OutView<Tr>& real,
-                                              double* __restrict__ norm, int p, int ut, int vt, unsigned* err) {
+                                              double* __restrict__ norm, int p, int ut, int vt, unsigned* err, int stall) {
     RsStageShared* sh = reinterpret_cast<RsStageShared*>(smem);
     float* stages = reinterpret_cast<float*>(smem + RSG_HEADER);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -332,7 +333,7 @@ __device__ __forceinline__ void rs_stage_tile(const DevGeom& g, const RsStageMap
     const int lo = sh->lo, hi = sh->hi;
     float acc = 0.f;
     if (warp >= 8) {
-        rsg_produce<Tv>(g, maps, stages, sh, turn, xm, upward, src, lo, hi, err);
+        rsg_produce<Tv>(g, maps, stages, sh, turn, xm, upward, src, lo, hi, err, stall);
     } else {
         const float dx = g.dx;
         const float2 SXY = make_float2(r.sx, r.sy);
@@ -352,11 +353,11 @@ __device__ __forceinline__ void rs_stage_tile(const DevGeom& g, const RsStageMap
             constexpr bool XM = decltype(axis)::value;
             for (bool more = lo <= hi; more;) {
                 const int s = turn % RSG_STAGES;
-                if (!mbar_wait(&sh->full[s], (turn / RSG_STAGES) & 1)) {
-                    atomicOr(err, ERR_TIMEOUT);
+                if (!mbar_wait_warp(&sh->full[s], (turn / RSG_STAGES) & 1)) {
+                    if (lane == 0) atomicOr(err, ERR_TIMEOUT);
                     break;
                 }
-                if (*(volatile int*)&sh->abort_flag) break;
+                if (__any_sync(0xffffffffu, *(volatile int*)&sh->abort_flag)) break;
                 const RsChunk ch = sh->chunk[s];
                 // samples before the chunk's edge; one within 0.1 of it waits for the next chunk,
                 // whose planes start one earlier

@@ -46,6 +46,11 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity
         }
     }
 }
+// The same for a whole warp: one answer for its 32 lanes, which may see the second pass at
+// different polls. All later control flow and __syncwarp() stay uniform over the warp.
+__device__ __forceinline__ bool mbar_wait_warp(unsigned long long* b, unsigned parity) {
+    return __all_sync(0xffffffffu, mbar_wait(b, parity));
+}
 __device__ __forceinline__ void tma_load_3d(float* dst, const CUtensorMap* map, int c0, int c1, int c2,
                                             unsigned long long* bar) {
     asm volatile(

@@ -367,10 +367,10 @@ void rs_stage_destroy(RsStage* t);
 cudaError_t rs_stage_fill(const void* vol, tomo_dtype vdt, int nx, int ny, int nz, const RsStage& t, cudaStream_t st,
                           const unsigned* amax = nullptr);
 size_t rs_stage_grid_blocks(const DevGeom& g);  // blocks of a launch (the EPI_NORM partials it writes)
-// Bounded waits report ERR_TIMEOUT in *err.
+// Bounded waits report ERR_TIMEOUT in *err (stall: as launch_vi_back_tma).
 cudaError_t launch_rs_stage(int mode, int epi, const DevGeom& g, const RsStage& t, unsigned long long tex,
                             const OutView<void>& out, tomo_dtype odt, const OutView<void>& real, tomo_dtype rdt, double* norm, unsigned* err,
-                            cudaStream_t st);
+                            cudaStream_t st, int stall = 0);
 void rs_tex_preload();
 int rs_tex_max_layers();
 // Elements of the RS input buffer for a layout, and the kernel that fills it from a volume.

@@ -115,7 +115,7 @@ __device__ __forceinline__ bool vi_tma_tile(const DevGeom& g, const CUtensorMap*
             for (int j = 0; j < min(32, g.np - pb); ++j) {
                 const int uj = __shfl_sync(0xffffffffu, u0, j), vj = __shfl_sync(0xffffffffu, v0, j);
                 const int s = turn.s;
-                if (!mbar_wait(&sh.empty[s], turn.phase ^ 1u)) {  // a fresh barrier counts as emptied
+                if (!mbar_wait_warp(&sh.empty[s], turn.phase ^ 1u)) {  // a fresh barrier counts as emptied
                     if (lane == 0) atomicOr(err, ERR_TIMEOUT);
                     alive = false;  // the consumers' waits run out as well
                     break;
@@ -140,7 +140,7 @@ __device__ __forceinline__ bool vi_tma_tile(const DevGeom& g, const CUtensorMap*
         // the copies in flight land before the block may exit
         VtTurn q = first;
         for (int p = 0; p < issued; ++p, q.next())
-            if (p >= issued - VT_STAGES && !mbar_wait(&sh.full[q.s], q.phase)) {
+            if (p >= issued - VT_STAGES && !mbar_wait_warp(&sh.full[q.s], q.phase)) {
                 if (lane == 0) atomicOr(err, ERR_TIMEOUT);
                 alive = false;
             }
@@ -187,8 +187,8 @@ __device__ __forceinline__ bool vi_tma_tile(const DevGeom& g, const CUtensorMap*
             fnum = fdiv(fmul(g.fdk_alpha, g.fdd_du), fmul(denum, denum));
             q0 = fmaf(up, up, g.fdk_beta);
         }
-        if (!mbar_wait(&sh.full[turn.s], turn.phase)) {
-            atomicOr(err, ERR_TIMEOUT);
+        if (!mbar_wait_warp(&sh.full[turn.s], turn.phase)) {
+            if (lane == 0) atomicOr(err, ERR_TIMEOUT);
             alive = false;
             break;
         }
