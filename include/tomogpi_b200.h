@@ -349,7 +349,12 @@ tomo_status tomo_batch_set_share(tomo_batch* b, double fraction);
 tomo_status tomo_batch_set_priority(tomo_batch* b, int32_t priority);
 /* Runs `count` iterations of every live job, ordered after the work already on `stream`. */
 tomo_status tomo_batch_iterate(tomo_batch* b, int32_t count, void* stream);
-/* Iterations a job has completed and its alpha_min (synchronises). */
+/* For tests of the bounded waits only, as tomo_context_test_stall: the batch's staged
+   backprojections issue no copies, their waits run out, and tomo_batch_job_status of the jobs
+   they served returns TOMO_ERR_TIMEOUT until those jobs are removed. */
+tomo_status tomo_batch_test_stall(tomo_batch* b, int enable);
+/* Iterations a job has completed and its alpha_min (synchronises). TOMO_ERR_TIMEOUT: a bounded
+   wait of one of the job's backprojections gave up, its iterate is undefined. */
 tomo_status tomo_batch_job_status(tomo_batch* b, int32_t job, int32_t* iterations_done, double* alpha_min,
                                   void* stream);
 tomo_status tomo_batch_job_alphas(tomo_batch* b, int32_t job, double* alpha, int32_t n, int32_t* written,

@@ -173,3 +173,33 @@ def test_batch_real_f32_matches_solver_and_mix():
     assert rel_l2(alone[0], solo) <= 1e-6
     rounded, _, _ = _run_batch([(cfg, g.to(torch.bfloat16))], _params(storage="bf16"), 4)
     assert not np.array_equal(rounded[0], alone[0])
+
+
+def test_batch_bounded_wait_is_reported_per_job():
+    """With the test stall the staged backprojection issues no copies and its waits run out: every
+    job that it served reports TOMO_ERR_TIMEOUT, a job added afterwards runs as always, and so
+    does the batch once the others are removed."""
+    import tomogpi_b200 as t
+    from tomogpi_b200 import _lib as L
+
+    jobs = [_job(n, 6, k) for k, n in enumerate((20, 33, 16))]
+    want = _run_batch([jobs[2]], _params(), 2)[0][0]
+    b = t.Batch(_params())
+    vols = [torch.zeros(cfg.volume_shape, device="cuda:0") for cfg, _ in jobs]
+    ids = [b.add(cfg, v, g) for (cfg, g), v in zip(jobs[:2], vols)]
+    L.call("tomo_batch_test_stall", b._h, 1)
+    b.iterate(1)
+    for i in ids:
+        with pytest.raises(L.TomoError, match="TIMEOUT"):
+            b.status(i)
+    L.call("tomo_batch_test_stall", b._h, 0)
+    ids.append(b.add(jobs[2][0], vols[2], jobs[2][1]))
+    b.iterate(2)
+    assert b.status(ids[2])[0] == 2
+    with pytest.raises(L.TomoError, match="TIMEOUT"):
+        b.status(ids[0])
+    for i in ids[:2]:
+        b.remove(i)
+    torch.cuda.synchronize()
+    assert np.array_equal(vols[2].cpu().numpy(), want)
+    b.close()

@@ -120,6 +120,7 @@ SIGNATURES = {
     "tomo_batch_set_graph": (ctypes.c_int, [_vp, ctypes.c_int]),
     "tomo_batch_set_share": (ctypes.c_int, [_vp, ctypes.c_double]),
     "tomo_batch_set_priority": (ctypes.c_int, [_vp, _i32]),
+    "tomo_batch_test_stall": (ctypes.c_int, [_vp, ctypes.c_int]),
     "tomo_batch_trim": (ctypes.c_int, [_vp, _vp]),
     "tomo_batch_host_times": (ctypes.c_int, [_vp, _vp]),
     "tomo_batch_iterate": (ctypes.c_int, [_vp, _i32, _vp]),

@@ -48,7 +48,7 @@ struct BatchJob {  // device descriptor of one job
     float* grad;
     double* part_proj;        // [P * UT * VT] partials of ||H dJ||^2
     double* part_lap;         // [2 * nz] partials of ||dJ||^2 and ||L dJ||^2
-    int* iter;                // next iteration (1-based)
+    int* iter;                // [0] next iteration (1-based), [1] amax, [2] error bits of the job's bounded waits
     unsigned* amax;           // FP16 storage: FP32 bits of max|dJ| (range guard), else null
     double* state;            // [0] alpha, [1] alpha_min, [2] 1 if the job stepped this iteration
     double* alpha_log;        // [iters]
@@ -178,13 +178,15 @@ __global__ void __launch_bounds__(VI_BX* VI_BY, vi_min_blocks(ZC)) batch_vi_kern
 }
 
 // The same with the detector windows staged by TMA (vi_tma.cuh), 16 slices per thread: jobs
-// whose residual is kept as rows. A wait that runs out stops the CTA and sets ERR_TIMEOUT.
+// whose residual is kept as rows. A wait that runs out stops the CTA and sets ERR_TIMEOUT in the
+// job's error bits; where every CTA stopped, the last one out sets it for the jobs whose items
+// nobody took (`out` counts the CTAs). stall: tests only (tomo_batch_test_stall).
 // Eight uneven BF16 jobs (64^3..192^3), two iterations: 32.0 -> 28.4 ms with this in place of
 // the zero-bordered form.
 template <int UM>
 __global__ void __launch_bounds__(VT_CONSUMERS + 32, 4) batch_vi_tma_kernel(const BatchJob* __restrict__ jobs, JobRanges r,
                                                                            int n_items, int* head, const int* share,
-                                                                           unsigned* err) {
+                                                                           int* out, int stall) {
     __shared__ VtShared<16> sh;
     vt_init(sh);
     VtTurn turn;
@@ -200,9 +202,18 @@ __global__ void __launch_bounds__(VT_CONSUMERS + 32, 4) batch_vi_tma_kernel(cons
         if (threadIdx.x >= VT_CONSUMERS) asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
         const int xt = (g.nx + VI_BX - 1) / VI_BX, yt = (g.ny + VI_BY - 1) / VI_BY;
         const long long t = local / xt;
-        const bool ok = vi_tma_tile<UM, 16, float, false>(g, map, J.resid, J.r_row, J.dJ, -2.0f, err, 0, sh, turn,
+        const bool ok = vi_tma_tile<UM, 16, float, false>(g, map, J.resid, J.r_row, J.dJ, -2.0f, (unsigned*)(J.iter + 2),
+                                                             stall, sh, turn,
                                                           (int)(local % xt), (int)(t % yt), (int)(t / yt));
         if (__syncthreads_or(!ok)) break;
+    }
+    __threadfence();  // this CTA's takes are counted before its departure
+    if (threadIdx.x == 0 && atomicAdd(out, 1) == (int)gridDim.x - 1) {
+        *out = 0;
+        const int taken = atomicAdd(head, 0);
+        for (int i = 0; i < r.n; ++i)
+            if (r.start[i + 1] > taken && job_active(jobs[r.job[i]]))
+                atomicOr((unsigned*)(jobs[r.job[i]].iter + 2), ERR_TIMEOUT);
     }
 }
 
@@ -426,7 +437,7 @@ struct tomo_batch {
     int n_jobs_dev = 0;
     std::vector<int> dev_to_slot;
     int* d_heads = nullptr;  // [0..2] residual projection per layout, [3..5] norm projection, [6..7] VI,
-                             // [8] CTA share of the persistent launches (per mille), [9] error bits
+                             // [8] CTA share of the persistent launches (per mille), [9] CTAs that have left
     cudaMemPool_t pool = nullptr;       // job buffers and tables: stream-ordered, so that adding or
                                         // retiring a job never waits for other streams' work
     cudaStream_t ctl_stream = nullptr;  // share updates, which must not queue behind own_stream
@@ -448,6 +459,7 @@ struct tomo_batch {
     cudaStream_t own_stream = nullptr;
     long long launches = 0;
     long long graph_launches = 0;
+    int test_stall = 0;  // tomo_batch_test_stall
     // A job-set change re-captures the iteration and updates the executable graph in place
     // (cudaGraphExecUpdate); executable graphs that could not be updated are destroyed only
     // at trim or destroy time, never while other streams run.
@@ -655,7 +667,7 @@ cudaError_t launch_batch_vi_group(tomo_batch* b, cudaStream_t st) {
         static int grid = 0;
         if (!grid) grid = persistent_grid(k, VT_CONSUMERS + 32, b->device);
         k<<<std::min(grid, n), VT_CONSUMERS + 32, 0, st>>>(b->d_jobs, b->ranges[3], n, b->d_heads + 6, b->d_heads + 8,
-                                                           (unsigned*)(b->d_heads + 9));
+                                                           b->d_heads + 9, b->test_stall);
         b->launches += 1;
         return cudaGetLastError();
     }
@@ -925,6 +937,13 @@ tomo_status tomo_batch_set_share(tomo_batch* b, double fraction) {
     return TOMO_OK;
 }
 
+tomo_status tomo_batch_test_stall(tomo_batch* b, int enable) {
+    TOMO_CHECK_ARG(b, "tomo_batch_test_stall: null argument");
+    b->test_stall = enable != 0;
+    b->recapture = true;  // a kernel parameter
+    return TOMO_OK;
+}
+
 tomo_status tomo_batch_set_priority(tomo_batch* b, int32_t priority) {
     TOMO_CHECK_ARG(b, "tomo_batch_set_priority: null argument");
     TOMO_CUDA_TRY(cudaSetDevice(b->device));
@@ -1022,18 +1041,16 @@ tomo_status tomo_batch_job_status(tomo_batch* b, int32_t job, int32_t* iteration
     TOMO_CUDA_TRY(cudaSetDevice(b->device));
     TOMO_CUDA_TRY(cudaStreamSynchronize((cudaStream_t)stream));
     TOMO_CUDA_TRY(cudaStreamSynchronize(b->own_stream));
-    int it = 0;
-    unsigned bits = 0;
+    int it[3] = {0, 0, 0};  // next iteration, amax, error bits
     double st[2] = {0, 0};
-    TOMO_CUDA_TRY(cudaMemcpyAsync(&bits, b->d_heads + 9, sizeof(bits), cudaMemcpyDeviceToHost, b->own_stream));
-    TOMO_CUDA_TRY(cudaMemcpyAsync(&it, b->jobs[job].d.iter, sizeof(int), cudaMemcpyDeviceToHost, b->own_stream));
+    TOMO_CUDA_TRY(cudaMemcpyAsync(it, b->jobs[job].d.iter, sizeof(it), cudaMemcpyDeviceToHost, b->own_stream));
     TOMO_CUDA_TRY(cudaMemcpyAsync(st, b->jobs[job].d.state, sizeof(st), cudaMemcpyDeviceToHost, b->own_stream));
     TOMO_CUDA_TRY(cudaStreamSynchronize(b->own_stream));
-    if (bits & ERR_TIMEOUT) {
-        set_error("tomo_batch: a bounded wait of the backprojection ran out");
-        return TOMO_ERR_CUDA;
+    if ((unsigned)it[2] & ERR_TIMEOUT) {
+        set_error("tomo_batch: a bounded wait of this job's backprojection ran out; its iterate is undefined");
+        return TOMO_ERR_TIMEOUT;
     }
-    *iterations_done = it - 1;
+    *iterations_done = it[0] - 1;
     if (alpha_min) *alpha_min = st[1];
     return TOMO_OK;
 }
