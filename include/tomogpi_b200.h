@@ -207,6 +207,10 @@ tomo_status tomo_context_errors(tomo_context* ctx, unsigned* bits, int clear);
    result undefined and bit 1 (a bounded wait gave up) set in the error word, and the
    context stays usable. Never enabled otherwise. */
 tomo_status tomo_context_test_stall(tomo_context* ctx, int enable);
+/* For tests of what happens without device memory only: after `skip` more device allocations
+   of the context and of its solvers, the next `count` are answered as out of memory, without
+   asking the device. */
+tomo_status tomo_context_test_deny(tomo_context* ctx, int32_t skip, int32_t count);
 
 /* ---- gradient descent (Iter3D::doSimpleGradient, src/TomoGPI_lib/src/CPP/Iter3D_Algo_Gradient.cu:25-223,
         and Iter3D::doWeightedGradient, :227-373; generalised-Gaussian regulariser

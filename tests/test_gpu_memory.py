@@ -1,0 +1,152 @@
+"""What contexts and solvers do when a device allocation fails: the staged forms' buffers are
+optional, so a call without room for them runs another form with the same result, and a call that
+fails leaves an object that can be used again. The failures are injected on the host
+(tomo_context_test_deny); nothing runs out of memory."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def tomo():
+    import tomogpi_b200 as t
+
+    return t
+
+
+def _deny(ctx, skip, count):
+    from tomogpi_b200 import _lib as L
+
+    L.call("tomo_context_test_deny", ctx.handle, skip, count)
+
+
+def _cfg(tomo, n=40, views=12):
+    return tomo.ConfigCT.cone_beam(n, views)
+
+
+def _volume(cfg, seed=1):
+    return torch.from_numpy(np.random.default_rng(seed).random(cfg.volume_shape, dtype=np.float32)).cuda()
+
+
+def _sino(cfg, seed=2):
+    return torch.from_numpy(np.random.default_rng(seed).random(cfg.sinogram_shape, dtype=np.float32)).cuda()
+
+
+def test_projection_without_room_for_the_copies(tomo):
+    """No room for the staged copies: the texture. Copies that give way to a later buffer: the
+    texture from then on. Bit-identical either way."""
+    cfg = _cfg(tomo)
+    vol = _volume(cfg)
+    with tomo.Context(cfg) as ctx:
+        ref = ctx.project("RS", vol)
+    with tomo.Context(cfg) as ctx:
+        _deny(ctx, 1, 1)  # after the projector's input buffer
+        assert torch.equal(ctx.project("RS", vol), ref)
+        assert torch.equal(ctx.project("RS", vol), ref)
+    with tomo.Context(cfg) as ctx:
+        ctx.project("RS", vol)
+        _deny(ctx, 0, 1)  # the host form's volume
+        assert np.array_equal(ctx.project_host("RS", vol.cpu().numpy()), ref.cpu().numpy())
+        assert torch.equal(ctx.project("RS", vol), ref)
+    with tomo.Context(cfg) as ctx:
+        _deny(ctx, 1, 2)  # neither the copies nor the texture
+        with pytest.raises(RuntimeError, match="NO_MEMORY"):
+            ctx.project("RS", vol)
+        assert torch.equal(ctx.project("RS", vol), ref)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_backprojection_without_room_for_the_rows(tomo, dtype):
+    """No room for the FP32 rows: the padded copy, bit-identical; nor for that one: an error, and
+    the next call runs."""
+    cfg = _cfg(tomo).replace(u_detector_pixel_nb=42)
+    s = _sino(cfg).to(dtype)
+    with tomo.Context(cfg) as ctx:
+        ref = ctx.backproject("VI", s, dtype=torch.float32)
+    with tomo.Context(cfg) as ctx:
+        _deny(ctx, 0, 2)
+        with pytest.raises(RuntimeError, match="NO_MEMORY"):
+            ctx.backproject("VI", s, dtype=torch.float32)
+        _deny(ctx, 0, 1)
+        assert torch.equal(ctx.backproject("VI", s, dtype=torch.float32), ref)
+        assert torch.equal(ctx.backproject("VI", s, dtype=torch.float32), ref)
+
+
+def _params(tomo, **kw):
+    return tomo.GradientParams(gradient_iteration_nb=2, optimal_step_iteration_nb=3, regularization_parameter=0.01, **kw)
+
+
+@pytest.mark.parametrize("storage", ["f32", "bf16"])
+def test_solver_creation_with_one_failed_allocation(tomo, storage):
+    """Whichever single allocation fails, creation reports it or the solver runs without it."""
+    cfg = _cfg(tomo)
+    s = _sino(cfg)
+    par = _params(tomo, storage=storage, real_f32=True)
+    with tomo.Context(cfg) as ctx:
+        ref = tomo.Solver(ctx, par).iterate(_volume(cfg), s).cpu().numpy()
+        made = 0
+        for skip in range(14):
+            _deny(ctx, skip, 1)
+            try:
+                sv = tomo.Solver(ctx, par)
+            except RuntimeError as e:
+                assert "NO_MEMORY" in str(e)
+                continue
+            _deny(ctx, 0, 0)
+            made += 1
+            assert rel_l2(sv.iterate(_volume(cfg), s).cpu().numpy(), ref) <= 1e-6, skip
+            sv.close()
+        assert made >= 2  # one without the failure at least
+
+
+@pytest.mark.parametrize("fails", [1, 2, 3, 4])
+@pytest.mark.parametrize("step", ["huber", "weights", "host"])
+def test_solver_whose_copies_gave_way(tomo, step, fails):
+    """A buffer that does not fit makes the solver's staged copies give way (1); the texture that
+    takes their place may not fit either (2), nor at the next iterations (3, 4). Every failing
+    call raises before it launches anything, and the solver then gives the same result."""
+    cfg = _cfg(tomo)
+    s = _sino(cfg)
+    w = torch.rand(cfg.sinogram_shape, device="cuda") + 0.5
+
+    def run(solver, deny):
+        tries = 0
+
+        def insist(f):
+            nonlocal tries
+            for _ in range(6):
+                try:
+                    return f()
+                except RuntimeError as e:
+                    assert "NO_MEMORY" in str(e)
+                    tries += 1
+            raise AssertionError("still no memory")
+
+        if deny:
+            _deny(solver.ctx, 0, deny)
+        if step == "host":
+            vol = _volume(cfg).cpu().numpy()
+            insist(lambda: solver.iterate_host(vol, s.cpu().numpy()))
+            return vol, tries
+        f = (lambda: solver.set_regularizer("huber", 0.02)) if step == "huber" else (lambda: solver.set_weights(w))
+        if deny >= 2:  # the failed call's buffer was not handed out; iterations go on without it
+            with pytest.raises(RuntimeError, match="NO_MEMORY"):
+                f()
+            tries += 1
+            insist(lambda: solver.iterate(_volume(cfg), s, first=1, count=0))
+            solver.set_state(-0.0347711, 1)
+        insist(f)
+        vol = _volume(cfg)
+        insist(lambda: solver.iterate(vol, s))
+        return vol.cpu().numpy(), tries
+
+    with tomo.Context(cfg) as ctx:
+        ref, none = run(tomo.Solver(ctx, _params(tomo)), 0)
+        got, tries = run(tomo.Solver(ctx, _params(tomo)), fails)
+        _deny(ctx, 0, 0)
+    assert none == 0 and (tries > 0) == (fails > 1)
+    assert rel_l2(got, ref) <= 1e-6

@@ -41,6 +41,7 @@ struct tomo_context {
     int* d_order = nullptr;
     unsigned* d_err = nullptr;
     int test_stall = 0;  // tomo_context_test_stall
+    int test_skip = 0, test_deny = 0;  // tomo_context_test_deny
     unsigned long long* d_count = nullptr;
     void* vpad[3] = {nullptr, nullptr, nullptr};  // padded volume per storage dtype
     void* spad[3] = {nullptr, nullptr, nullptr};  // padded sinogram per storage dtype
@@ -125,39 +126,58 @@ std::pair<cudaEvent_t, cudaEvent_t>* next_events(std::vector<std::pair<cudaEvent
 
 namespace {
 
-tomo_status ensure(void** p, size_t bytes, bool zero) {
+// Tests only: whether this device allocation of the context or of its solvers is to fail.
+bool test_denied(tomo_context* ctx) {
+    if (ctx->test_skip > 0) {
+        --ctx->test_skip;
+        return false;
+    }
+    return ctx->test_deny > 0 && ctx->test_deny-- > 0;
+}
+
+tomo_status alloc_once(tomo_context* ctx, void** p, size_t bytes, bool zero) {
     if (*p) return TOMO_OK;
-    TOMO_CUDA_TRY(cudaMalloc(p, bytes));
+    const cudaError_t e = test_denied(ctx) ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        return cuda_fail(e, "cudaMalloc");
+    }
     if (zero) TOMO_CUDA_TRY(cudaMemset(*p, 0, bytes));
     return TOMO_OK;
 }
 
-// The same for a context's or solver's buffers: its staged copies give way to them (its
-// projections then gather from the texture, half the size in FP32).
-tomo_status ensure_beside(RsStage* stage, void** p, size_t bytes, bool zero) {
-    const tomo_status s = ensure(p, bytes, zero);
-    if (s != TOMO_ERR_NO_MEMORY || !stage->rows) return s;
+// A buffer of the context's: its staged copies give way to it (its projections then gather from
+// the texture, half the size in FP32).
+tomo_status ensure(tomo_context* ctx, void** p, size_t bytes, bool zero) {
+    const tomo_status s = alloc_once(ctx, p, bytes, zero);
+    if (s != TOMO_ERR_NO_MEMORY || !ctx->stage.rows) return s;
     cudaGetLastError();
     TOMO_CUDA_TRY(cudaDeviceSynchronize());
-    rs_stage_destroy(stage);
-    return ensure(p, bytes, zero);
+    rs_stage_destroy(&ctx->stage);
+    ctx->stage_denied = true;
+    return alloc_once(ctx, p, bytes, zero);
 }
-tomo_status ensure(tomo_context* ctx, void** p, size_t bytes, bool zero) {
-    const bool staged = ctx->stage.rows != nullptr;
-    const tomo_status s = ensure_beside(&ctx->stage, p, bytes, zero);
-    if (staged && !ctx->stage.rows) ctx->stage_denied = true;
-    return s;
-}
-cudaError_t solver_texture(tomo_solver* sv) {
+
+tomo_status solver_texture(tomo_solver* sv) {
     const HostGeom& h = sv->ctx->hg;
-    const cudaError_t e = rs_vol_tex_create(h.nx, h.ny, h.nz, sv->prm.storage, &sv->tex, 0);
-    return e == cudaSuccess ? cudaStreamSynchronize(0) : e;  // creation only: the zero layers are written
+    const cudaError_t e = test_denied(sv->ctx) ? cudaErrorMemoryAllocation
+                                               : rs_vol_tex_create(h.nx, h.ny, h.nz, sv->prm.storage, &sv->tex, 0);
+    if (e != cudaSuccess) return cuda_fail(e, "rs texture");
+    TOMO_CUDA_TRY(cudaStreamSynchronize(0));  // creation only: the zero layers are written
+    return TOMO_OK;
 }
+
+// A buffer of the solver's: its staged copies give way to it. The texture that takes their
+// place is made before the buffer; without room for it the solver has neither until solver_run
+// makes it, and the buffer is not handed out.
 tomo_status ensure(tomo_solver* sv, void** p, size_t bytes, bool zero) {
-    const bool staged = sv->stage.rows != nullptr;
-    const tomo_status s = ensure_beside(&sv->stage, p, bytes, zero);
-    if (staged && !sv->stage.rows && !sv->tex.tex) TOMO_CUDA_TRY(solver_texture(sv));
-    return s;
+    tomo_status s = alloc_once(sv->ctx, p, bytes, zero);
+    if (s != TOMO_ERR_NO_MEMORY || !sv->stage.rows) return s;
+    cudaGetLastError();
+    TOMO_CUDA_TRY(cudaDeviceSynchronize());
+    rs_stage_destroy(&sv->stage);
+    if (!sv->tex.tex && (s = solver_texture(sv)) != TOMO_OK) return s;
+    return alloc_once(sv->ctx, p, bytes, zero);
 }
 
 tomo_status set_device(const tomo_context* ctx) {
@@ -228,8 +248,9 @@ tomo_status context_texture(tomo_context* ctx, bool march, const void* vol, tomo
             TOMO_CUDA_TRY(cudaStreamSynchronize(st));
             rs_tex_destroy(&ctx->tex);
         }
-        const cudaError_t e = march ? rs_march_tex_create(g.nx, g.ny, g.nz, &ctx->tex)
-                                    : rs_vol_tex_create(g.nx, g.ny, g.nz, vdt, &ctx->tex, st);
+        const cudaError_t e = test_denied(ctx) ? cudaErrorMemoryAllocation
+                              : march          ? rs_march_tex_create(g.nx, g.ny, g.nz, &ctx->tex)
+                                               : rs_vol_tex_create(g.nx, g.ny, g.nz, vdt, &ctx->tex, st);
         if (e != cudaSuccess) return cuda_fail(e, "rs texture");
     }
     return check_launch(rs_tex_fill(vol, vdt, g.nx, g.ny, g.nz, ctx->tex, st), "rs texture fill");
@@ -252,7 +273,9 @@ tomo_status project_into(tomo_context* ctx, tomo_projector kind, const void* vol
                 TOMO_CUDA_TRY(cudaStreamSynchronize(st));
                 rs_stage_destroy(&ctx->stage);
             }
-            cudaError_t e = ctx->stage.rows ? cudaSuccess : rs_stage_create(g.nx, g.ny, g.nz, vdt, &ctx->stage);
+            const cudaError_t e = ctx->stage.rows    ? cudaSuccess
+                                  : test_denied(ctx) ? cudaErrorMemoryAllocation
+                                                     : rs_stage_create(g.nx, g.ny, g.nz, vdt, &ctx->stage);
             if (e == cudaErrorMemoryAllocation) {  // no memory for the copies: the texture alone
                 ctx->stage_denied = true;
                 staged = false;
@@ -472,10 +495,7 @@ tomo_status tomo_backproject(tomo_context* ctx, tomo_backprojector kind, const v
         long pitch = g.nu;
         if (sinogram_dtype != TOMO_F32 || !vi_tma_supported(sinogram, g.nu)) {
             pitch = vi_rows_pitch(g.nu);
-            if (!ctx->rows && cudaMalloc((void**)&ctx->rows, (size_t)pitch * g.nv * g.np * sizeof(float)) != cudaSuccess) {
-                cudaGetLastError();
-                ctx->rows = nullptr;
-            }
+            if (alloc_once(ctx, (void**)&ctx->rows, ctx->nsino_rows() * sizeof(float), false) != TOMO_OK) cudaGetLastError();
             rows = ctx->rows;
             if (rows && (s = check_launch(launch_sino_rows(sinogram, sinogram_dtype, ctx->rows, g.nu, g.nv, g.np, (int)pitch, st),
                                           "sinogram rows")) != TOMO_OK)
@@ -629,6 +649,13 @@ tomo_status tomo_context_test_stall(tomo_context* ctx, int enable) {
     return TOMO_OK;
 }
 
+tomo_status tomo_context_test_deny(tomo_context* ctx, int32_t skip, int32_t count) {
+    TOMO_CHECK_ARG(ctx && skip >= 0 && count >= 0, "tomo_context_test_deny: bad argument");
+    ctx->test_skip = skip;
+    ctx->test_deny = count;
+    return TOMO_OK;
+}
+
 // ------------------------------------------------------------------------------------
 // Gradient solver.
 // ------------------------------------------------------------------------------------
@@ -651,9 +678,7 @@ tomo_status tomo_solver_create(tomo_context* ctx, const tomo_gradient_params* pr
     sv->log_cap = prm->gradient_iteration_nb > 0 ? prm->gradient_iteration_nb : 1;
     const size_t es = dtype_size(prm->storage);
     auto alloc = [&](void** p, size_t bytes, bool zero) -> bool {
-        if (cudaMalloc(p, bytes) != cudaSuccess) return false;
-        if (zero && cudaMemset(*p, 0, bytes) != cudaSuccess) return false;
-        return true;
+        return alloc_once(ctx, p, bytes, zero) == TOMO_OK;
     };
     bool ok = alloc(&sv->vpad, rs_input_elems(sv->rs_layout, ctx->hg.nx, ctx->hg.ny, ctx->hg.nz) * es, true) && alloc(&sv->spad, std::max(ctx->nsino_pad(), ctx->nsino_rows()) * sizeof(float), true) &&
               alloc((void**)&sv->dJ, ctx->nvox() * sizeof(float), false) &&
@@ -666,7 +691,7 @@ tomo_status tomo_solver_create(tomo_context* ctx, const tomo_gradient_params* pr
     const bool staged = rs && sv->rs_layout == RS_LAYOUT_TEX && rs_stage_supported(ctx->g, prm->storage);
     if (ok && !(staged && prm->storage == TOMO_F32) &&
         (sv->rs_layout == RS_LAYOUT_TEX || sv->rs_layout == RS_LAYOUT_HYBRID))
-        ok = solver_texture(sv) == cudaSuccess;
+        ok = solver_texture(sv) == TOMO_OK;
     if (ok) {  // the norm projection's per-block partials (the launch shape is fixed by now)
         const bool sid = prm->projector == TOMO_PROJ_SIDDON || prm->projector == TOMO_PROJ_SIDDON_REF;
         sv->npartials = sid ? siddon_grid_blocks(ctx->g) : rs_grid_blocks(sv->rs_layout, ctx->g);
@@ -681,9 +706,10 @@ tomo_status tomo_solver_create(tomo_context* ctx, const tomo_gradient_params* pr
         ok = rs_tex_create(ctx->hg.nu, ctx->hg.nv, ctx->hg.np, TOMO_F32, &sv->vtex, true) == cudaSuccess;
     if (ok) sv->vi_tma = !sv->vtex.tex && vi_staged(ctx);
     // last, and given back when a later allocation needs the room (ensure)
-    if (ok && staged && rs_stage_create(ctx->hg.nx, ctx->hg.ny, ctx->hg.nz, prm->storage, &sv->stage) != cudaSuccess) {
+    if (ok && staged &&
+        (test_denied(ctx) || rs_stage_create(ctx->hg.nx, ctx->hg.ny, ctx->hg.nz, prm->storage, &sv->stage) != cudaSuccess)) {
         cudaGetLastError();  // no memory for the copies: the texture alone
-        ok = sv->tex.tex || solver_texture(sv) == cudaSuccess;
+        ok = sv->tex.tex || solver_texture(sv) == TOMO_OK;
     }
     if (!ok) {
         cudaGetLastError();
@@ -738,7 +764,6 @@ tomo_status tomo_solver_set_regularizer(tomo_solver* sv, int32_t kind, double hu
         TOMO_CUDA_TRY(cudaSetDevice(sv->device));
         if (ensure(sv, (void**)&sv->htmp, sv->ctx->nvox() * sizeof(float), false) != TOMO_OK) {
             cudaGetLastError();
-            sv->htmp = nullptr;
             set_error("tomo_solver_set_regularizer: device allocation failed");
             return TOMO_ERR_NO_MEMORY;
         }
@@ -800,6 +825,10 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
     const OutView<void> resid = sv->vi_tma ? rows_view(sv->spad, h) : padded_view(sv->spad, h);
     const OutView<void> realv = plain_view(const_cast<void*>(real_sinogram), h);
     const bool siddon = P.projector == TOMO_PROJ_SIDDON || P.projector == TOMO_PROJ_SIDDON_REF;
+    // copies that gave way to a buffer while there was no room for the texture (ensure)
+    if (!siddon && sv->rs_layout == RS_LAYOUT_TEX && !sv->stage.rows && !sv->tex.tex &&
+        (s = solver_texture(sv)) != TOMO_OK)
+        return s;
     const size_t nparts = siddon           ? siddon_grid_blocks(g)
                           : sv->stage.rows ? rs_stage_grid_blocks(g)
                                            : rs_grid_blocks(sv->rs_layout, g);
