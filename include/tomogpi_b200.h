@@ -171,8 +171,8 @@ tomo_status tomo_backproject_host(tomo_context* ctx, tomo_backprojector kind, co
 /* Ramp filter of filtered backprojection (Matlab/Tomo8/ramp_filter_TOMO8.m: ramp over
    oversampling x nu frequencies, Hann window of cutoff x that length, convolution of every
    detector row, / (2 du)); the reference calls it with oversampling 16 and cutoff 1.0.
-   `out` is an FP32 device sinogram; the taps are cached in the context per (oversampling,
-   cutoff). */
+   `out` is an FP32 device sinogram, which may be the (FP32) input for rows of up to 6144
+   pixels; the taps are cached in the context per (oversampling, cutoff). */
 tomo_status tomo_ramp_filter(tomo_context* ctx, const void* sinogram, tomo_dtype sinogram_dtype, float* out,
                              int32_t oversampling, double cutoff, void* stream);
 /* The same on host FP32 buffers (out may be the input). */
