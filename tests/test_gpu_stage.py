@@ -168,3 +168,32 @@ def test_staged_projection_bounded_wait_reports_timeout(tomo, dtype, n, views):
         L.call("tomo_context_test_stall", ctx.handle, 0)
         assert torch.equal(ctx.project("RS", vol), ref)
         assert ctx.errors() == 0
+
+
+def test_copies_of_many_contexts_threads_and_streams(tomo):
+    """The copies' memory outlives a context in its device's pool: contexts of several sizes, made
+    and closed by four threads on streams of their own, each see their own copies."""
+    import concurrent.futures as cf
+
+    cfgs = [_cfg(tomo, n, n, n, n, n, 12, 2.0) for n in (40, 64, 100, 128)]
+    vols = [torch.rand(c.volume_shape, device="cuda") for c in cfgs]
+    refs = []
+    for c, v in zip(cfgs, vols):
+        with tomo.Context(c) as ctx:
+            ctx.set_tuning(rs_layout="plain")
+            refs.append(ctx.project("RS", v))
+    torch.cuda.synchronize()
+
+    def work(k):
+        st, good = torch.cuda.Stream(), 0
+        with torch.cuda.stream(st):
+            for i in range(12):
+                j = (k + i) % len(cfgs)
+                with tomo.Context(cfgs[j]) as ctx:
+                    out = ctx.project("RS", vols[j])
+                    st.synchronize()
+                    good += int(torch.equal(out, refs[j]))
+        return good
+
+    with cf.ThreadPoolExecutor(4) as ex:
+        assert list(ex.map(work, range(4))) == [12] * 4

@@ -137,7 +137,15 @@ bool test_denied(tomo_context* ctx) {
 
 tomo_status alloc_once(tomo_context* ctx, void** p, size_t bytes, bool zero) {
     if (*p) return TOMO_OK;
-    const cudaError_t e = test_denied(ctx) ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
+    cudaError_t e = cudaErrorMemoryAllocation;
+    if (!test_denied(ctx)) {
+        e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            rs_stage_trim(ctx->device);
+            e = cudaMalloc(p, bytes);
+        }
+    }
     if (e != cudaSuccess) {
         *p = nullptr;
         return cuda_fail(e, "cudaMalloc");
@@ -154,6 +162,7 @@ tomo_status ensure(tomo_context* ctx, void** p, size_t bytes, bool zero) {
     cudaGetLastError();
     TOMO_CUDA_TRY(cudaDeviceSynchronize());
     rs_stage_destroy(&ctx->stage);
+    rs_stage_trim(ctx->device);
     ctx->stage_denied = true;
     return alloc_once(ctx, p, bytes, zero);
 }
@@ -176,6 +185,7 @@ tomo_status ensure(tomo_solver* sv, void** p, size_t bytes, bool zero) {
     cudaGetLastError();
     TOMO_CUDA_TRY(cudaDeviceSynchronize());
     rs_stage_destroy(&sv->stage);
+    rs_stage_trim(sv->device);
     if (!sv->tex.tex && (s = solver_texture(sv)) != TOMO_OK) return s;
     return alloc_once(sv->ctx, p, bytes, zero);
 }

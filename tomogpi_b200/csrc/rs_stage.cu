@@ -2,6 +2,7 @@
 // kernel, the two volume copies that it reads and their tensor maps.
 #include <algorithm>
 #include <atomic>
+#include <mutex>
 #include <new>
 
 #include "rs_stage.cuh"
@@ -84,6 +85,50 @@ bool rs_stage_supported(const DevGeom& g, tomo_dtype dt) {
     return vox >= 2097152.0 && samples >= 40.0 * vox;
 }
 
+// Copies of up to 64 MiB come from a pool of their device that keeps as much of what is freed, so
+// that small jobs, one context after another, do not pay the driver's allocation each time (a
+// context's first FP32 projection, 64^3, 60 views: 110 us, 420 with cudaMalloc). Larger ones
+// are cudaMalloc's: at 384^3 2.5 ms from the pool, 0.4. Pool memory is allocated and released
+// on a stream of the pool's on which nothing else runs.
+constexpr size_t POOL_KEEP = 64u << 20;
+struct StagePool {
+    std::mutex mu;
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t st = nullptr;
+};
+static StagePool* stage_pool(int dev) {
+    static StagePool pools[64];
+    return dev >= 0 && dev < 64 ? &pools[dev] : nullptr;
+}
+static cudaError_t pool_alloc(void** p, size_t bytes, int dev) {
+    StagePool* sp = stage_pool(dev);
+    if (!sp) return cudaErrorMemoryAllocation;
+    {
+        std::lock_guard<std::mutex> lock(sp->mu);
+        cudaError_t e = cudaSuccess;
+        if (!sp->st) e = cudaStreamCreateWithFlags(&sp->st, cudaStreamNonBlocking);
+        if (e == cudaSuccess && !sp->pool) {
+            cudaMemPoolProps pp{};
+            pp.allocType = cudaMemAllocationTypePinned;
+            pp.location.type = cudaMemLocationTypeDevice;
+            pp.location.id = dev;
+            unsigned long long keep = POOL_KEEP;
+            e = cudaMemPoolCreate(&sp->pool, &pp);
+            if (e == cudaSuccess) e = cudaMemPoolSetAttribute(sp->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        }
+        if (e != cudaSuccess) return e;
+    }
+    const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, sp->pool, sp->st);
+    return e == cudaSuccess ? cudaStreamSynchronize(sp->st) : e;  // usable from any stream
+}
+
+void rs_stage_trim(int dev) {
+    StagePool* sp = stage_pool(dev);
+    if (!sp) return;
+    std::lock_guard<std::mutex> lock(sp->mu);
+    if (sp->pool) cudaMemPoolTrimTo(sp->pool, 0);
+}
+
 cudaError_t rs_stage_create(int nx, int ny, int nz, tomo_dtype dt, RsStage* t) {
     *t = RsStage();
     const int nzr = stage_slices(dt, nz);
@@ -91,7 +136,9 @@ cudaError_t rs_stage_create(int nx, int ny, int nz, tomo_dtype dt, RsStage* t) {
     // one allocation: rows, then cols from a 256-byte boundary
     const size_t rb = ((size_t)nzr * ny * px * 4 + 255) & ~(size_t)255, cb = (size_t)nzr * nx * py * 4;
     char* base = nullptr;
-    cudaError_t e = cudaMalloc((void**)&base, rb + cb);
+    cudaError_t e = cudaGetDevice(&t->device);
+    t->pooled = rb + cb <= POOL_KEEP;
+    if (e == cudaSuccess) e = t->pooled ? pool_alloc((void**)&base, rb + cb, t->device) : cudaMalloc((void**)&base, rb + cb);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return e;
@@ -128,7 +175,16 @@ cudaError_t rs_stage_create(int nx, int ny, int nz, tomo_dtype dt, RsStage* t) {
 }
 
 void rs_stage_destroy(RsStage* t) {
-    cudaFree(t->rows);  // the one allocation
+    if (t->rows && t->pooled) {
+        // the launches that read the copies may be on any stream; where they cannot be waited for
+        // (another thread captures) the memory is not reused
+        if (cudaDeviceSynchronize() == cudaSuccess) {
+            cudaFreeAsync(t->rows, stage_pool(t->device)->st);
+            cudaStreamSynchronize(stage_pool(t->device)->st);
+        }
+    } else {
+        cudaFree(t->rows);  // the one allocation
+    }
     delete t->maps;
     *t = RsStage();
 }

@@ -359,10 +359,13 @@ struct RsStage {
     RsStageMaps* maps = nullptr;  // host memory: a launch takes them by value
     tomo_dtype dt = TOMO_F32;
     int px = 0, py = 0;  // row pitches of the copies, in words
+    int device = 0;      // current when they are made and destroyed
+    bool pooled = false; // from the device's pool
 };
 bool rs_stage_supported(const DevGeom& g, tomo_dtype dt);
 cudaError_t rs_stage_create(int nx, int ny, int nz, tomo_dtype dt, RsStage* t);
 void rs_stage_destroy(RsStage* t);
+void rs_stage_trim(int device);  // gives back what freed copies left in the device's pool
 // Fills the copies from a dense device volume (FP32, or of the copies' type).
 cudaError_t rs_stage_fill(const void* vol, tomo_dtype vdt, int nx, int ny, int nz, const RsStage& t, cudaStream_t st,
                           const unsigned* amax = nullptr);
