@@ -150,3 +150,65 @@ def test_solver_whose_copies_gave_way(tomo, step, fails):
         _deny(ctx, 0, 0)
     assert none == 0 and (tries > 0) == (fails > 1)
     assert rel_l2(got, ref) <= 1e-6
+
+
+def _captured(f):
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        f()
+    return g
+
+
+def test_captured_launches_keep_their_buffers(tomo):
+    """The copies and rows that a captured projection or backprojection reads never give way, to a
+    buffer or to a volume of another type: the replay is exact after either."""
+    cfg = _cfg(tomo, n=128, views=45).replace(u_detector_pixel_nb=126)
+    vol, s = _volume(cfg), _sino(cfg).to(torch.bfloat16)
+    with tomo.Context(cfg) as ctx:
+        fwd, back = ctx.project("RS", vol), ctx.backproject("VI", s, dtype=torch.float32)
+        ref, bref = fwd.clone(), back.clone()
+        g = _captured(lambda: (ctx.project("RS", vol, out=fwd), ctx.backproject("VI", s, out=back)))
+        _deny(ctx, 0, 1)
+        with pytest.raises(RuntimeError, match="NO_MEMORY"):
+            ctx.project_host("RS", vol.cpu().numpy())
+        half = ctx.project("RS", vol.to(torch.bfloat16), dtype=torch.float32)
+        fwd.zero_(), back.zero_()
+        g.replay()
+        assert torch.equal(fwd, ref) and torch.equal(back, bref)
+        ctx.set_tuning(rs_layout="cell8")
+        assert torch.equal(half, ctx.project("RS", vol.to(torch.bfloat16), dtype=torch.float32))
+        torch.cuda.synchronize()
+        del g
+
+
+def test_captured_iterations_keep_the_solvers_copies(tomo):
+    """The same for the copies that a solver's captured iterations read."""
+    cfg = _cfg(tomo)
+    s = _sino(cfg)
+    with tomo.Context(cfg) as ctx:
+        sv = tomo.Solver(ctx, _params(tomo))
+        vol = _volume(cfg)
+        ref = sv.iterate(vol, s).clone()
+        g = _captured(lambda: sv.iterate(vol, s))
+        _deny(ctx, 0, 1)
+        with pytest.raises(RuntimeError, match="NO_MEMORY"):
+            sv.set_regularizer("huber", 0.02)
+        sv.set_state(-0.0347711, 1)
+        vol.copy_(_volume(cfg))
+        g.replay()
+        assert rel_l2(vol.cpu().numpy(), ref.cpu().numpy()) <= 1e-6
+        torch.cuda.synchronize()
+        del g
+
+
+def test_copies_give_way_to_a_new_solver(tomo):
+    """A solver that finds no room takes that of the context's copies and rows."""
+    cfg = _cfg(tomo).replace(u_detector_pixel_nb=42)
+    vol, s = _volume(cfg), _sino(cfg)
+    with tomo.Context(cfg) as ctx:
+        ref = tomo.Solver(ctx, _params(tomo)).iterate(vol.clone(), s)
+    with tomo.Context(cfg) as ctx:
+        fwd, back = ctx.project("RS", vol), ctx.backproject("VI", s)
+        _deny(ctx, 1, 1)
+        assert rel_l2(tomo.Solver(ctx, _params(tomo)).iterate(vol.clone(), s).cpu().numpy(), ref.cpu().numpy()) <= 1e-6
+        assert torch.equal(ctx.project("RS", vol), fwd) and torch.equal(ctx.backproject("VI", s), back)

@@ -56,6 +56,7 @@ struct tomo_context {
     RsTexture tex;                       // TEX layout: layered array of the volume's type
     RsStage stage;                       // TEX layout, staged: the volume's copies
     bool stage_denied = false;           // no memory for them: the texture instead
+    bool stage_held = false, rows_held = false;  // a captured launch reads them: kept as long as the context
     RsTexture vtex;                      // VI texture layout: layered array of the sinogram
     float* d_ramp = nullptr;             // ramp-filter taps for (ramp_over, ramp_cut)
     int ramp_half = 0, ramp_over = 0;
@@ -93,6 +94,7 @@ struct tomo_solver {
     int next_it = 1;
     RsTexture tex;   // TEX layout resources of this solver (storage type)
     RsStage stage;   // ... or, where the geometry allows staging, these
+    bool stage_held = false;  // a captured launch reads them
     RsTexture vtex;  // VI texture layout: the FP32 residual, one layer per view
     bool vi_tma = false;  // VI through TMA-staged windows: the residual is kept plain, not padded
     // host-buffer form
@@ -154,34 +156,59 @@ tomo_status alloc_once(tomo_context* ctx, void** p, size_t bytes, bool zero) {
     return TOMO_OK;
 }
 
-// A buffer of the context's: its staged copies give way to it (its projections then gather from
-// the texture, half the size in FP32).
+bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &c) != cudaSuccess) cudaGetLastError();
+    return c != cudaStreamCaptureStatusNone;
+}
+
+// Makes room for another buffer: frees what the context's projections and backprojections can do
+// without (their staged copies, for the texture, half the size in FP32; their rows, for the padded
+// copy), unless a captured launch reads it. Whether anything was freed.
+bool give_way(tomo_context* ctx) {
+    const bool stage = ctx->stage.rows && !ctx->stage_held, rows = ctx->rows && !ctx->rows_held;
+    cudaGetLastError();
+    if ((!stage && !rows) || cudaDeviceSynchronize() != cudaSuccess) return false;
+    if (stage) {
+        rs_stage_destroy(&ctx->stage);
+        rs_stage_trim(ctx->device);
+        ctx->stage_denied = true;
+    }
+    if (rows) {
+        cudaFree(ctx->rows);
+        ctx->rows = nullptr;
+    }
+    return true;
+}
+
+// A buffer of the context's, or of a solver's as it is created.
 tomo_status ensure(tomo_context* ctx, void** p, size_t bytes, bool zero) {
     const tomo_status s = alloc_once(ctx, p, bytes, zero);
-    if (s != TOMO_ERR_NO_MEMORY || !ctx->stage.rows) return s;
-    cudaGetLastError();
-    TOMO_CUDA_TRY(cudaDeviceSynchronize());
-    rs_stage_destroy(&ctx->stage);
-    rs_stage_trim(ctx->device);
-    ctx->stage_denied = true;
-    return alloc_once(ctx, p, bytes, zero);
+    return s == TOMO_ERR_NO_MEMORY && give_way(ctx) ? alloc_once(ctx, p, bytes, zero) : s;
+}
+// The same for a texture that `make` creates.
+template <typename F>
+cudaError_t ensure_texture(tomo_context* ctx, F make) {
+    auto once = [&] { return test_denied(ctx) ? cudaErrorMemoryAllocation : make(); };
+    const cudaError_t e = once();
+    return e == cudaErrorMemoryAllocation && give_way(ctx) ? once() : e;
 }
 
 tomo_status solver_texture(tomo_solver* sv) {
     const HostGeom& h = sv->ctx->hg;
-    const cudaError_t e = test_denied(sv->ctx) ? cudaErrorMemoryAllocation
-                                               : rs_vol_tex_create(h.nx, h.ny, h.nz, sv->prm.storage, &sv->tex, 0);
+    const cudaError_t e =
+        ensure_texture(sv->ctx, [&] { return rs_vol_tex_create(h.nx, h.ny, h.nz, sv->prm.storage, &sv->tex, 0); });
     if (e != cudaSuccess) return cuda_fail(e, "rs texture");
     TOMO_CUDA_TRY(cudaStreamSynchronize(0));  // creation only: the zero layers are written
     return TOMO_OK;
 }
 
-// A buffer of the solver's: its staged copies give way to it. The texture that takes their
+// A buffer of the solver's: the context's and its own staged copies give way to it. The texture that takes their
 // place is made before the buffer; without room for it the solver has neither until solver_run
 // makes it, and the buffer is not handed out.
 tomo_status ensure(tomo_solver* sv, void** p, size_t bytes, bool zero) {
-    tomo_status s = alloc_once(sv->ctx, p, bytes, zero);
-    if (s != TOMO_ERR_NO_MEMORY || !sv->stage.rows) return s;
+    tomo_status s = ensure(sv->ctx, p, bytes, zero);
+    if (s != TOMO_ERR_NO_MEMORY || !sv->stage.rows || sv->stage_held) return s;
     cudaGetLastError();
     TOMO_CUDA_TRY(cudaDeviceSynchronize());
     rs_stage_destroy(&sv->stage);
@@ -258,9 +285,10 @@ tomo_status context_texture(tomo_context* ctx, bool march, const void* vol, tomo
             TOMO_CUDA_TRY(cudaStreamSynchronize(st));
             rs_tex_destroy(&ctx->tex);
         }
-        const cudaError_t e = test_denied(ctx) ? cudaErrorMemoryAllocation
-                              : march          ? rs_march_tex_create(g.nx, g.ny, g.nz, &ctx->tex)
-                                               : rs_vol_tex_create(g.nx, g.ny, g.nz, vdt, &ctx->tex, st);
+        const cudaError_t e = ensure_texture(ctx, [&] {
+            return march ? rs_march_tex_create(g.nx, g.ny, g.nz, &ctx->tex)
+                         : rs_vol_tex_create(g.nx, g.ny, g.nz, vdt, &ctx->tex, st);
+        });
         if (e != cudaSuccess) return cuda_fail(e, "rs texture");
     }
     return check_launch(rs_tex_fill(vol, vdt, g.nx, g.ny, g.nz, ctx->tex, st), "rs texture fill");
@@ -274,15 +302,19 @@ tomo_status project_into(tomo_context* ctx, tomo_projector kind, const void* vol
     if (kind == TOMO_PROJ_RS || kind == TOMO_PROJ_RS_UM) {
         const int layout = effective_layout(ctx->tuning.rs_layout, vdt, g.nx, g.ny, g.nz);
         bool staged = layout == RS_LAYOUT_TEX && !ctx->stage_denied && rs_stage_supported(g, vdt);
+        if (staged && ctx->stage.rows && ctx->stage.dt != vdt) {  // copies of another type
+            if (ctx->stage_held) {
+                staged = false;
+            } else {
+                TOMO_CUDA_TRY(cudaStreamSynchronize(st));
+                rs_stage_destroy(&ctx->stage);
+            }
+        }
         if (layout == RS_LAYOUT_HYBRID || layout == RS_LAYOUT_MARCH || (layout == RS_LAYOUT_TEX && !(staged && vdt == TOMO_F32))) {
             const tomo_status s = context_texture(ctx, layout == RS_LAYOUT_MARCH, vol, vdt, st);
             if (s != TOMO_OK) return s;
         }
         if (staged) {
-            if (ctx->stage.rows && ctx->stage.dt != vdt) {
-                TOMO_CUDA_TRY(cudaStreamSynchronize(st));
-                rs_stage_destroy(&ctx->stage);
-            }
             const cudaError_t e = ctx->stage.rows    ? cudaSuccess
                                   : test_denied(ctx) ? cudaErrorMemoryAllocation
                                                      : rs_stage_create(g.nx, g.ny, g.nz, vdt, &ctx->stage);
@@ -296,6 +328,7 @@ tomo_status project_into(tomo_context* ctx, tomo_projector kind, const void* vol
             }
         }
         if (staged) {
+            if (!ctx->stage_held) ctx->stage_held = capturing(st);
             const tomo_status s = check_launch(rs_stage_fill(vol, vdt, g.nx, g.ny, g.nz, ctx->stage, st), "rs stage fill");
             if (s != TOMO_OK) return s;
             return check_launch(launch_rs_stage(kind == TOMO_PROJ_RS ? 0 : 1, epi, g, ctx->stage, ctx->tex.tex, out, odt, real,
@@ -488,7 +521,8 @@ tomo_status tomo_backproject(tomo_context* ctx, tomo_backprojector kind, const v
                 TOMO_CUDA_TRY(cudaStreamSynchronize(st));
                 rs_tex_destroy(&ctx->vtex);
             }
-            cudaError_t e = rs_tex_create(g.nu, g.nv, g.np, sinogram_dtype, &ctx->vtex);
+            const cudaError_t e =
+                ensure_texture(ctx, [&] { return rs_tex_create(g.nu, g.nv, g.np, sinogram_dtype, &ctx->vtex); });
             if (e != cudaSuccess) return cuda_fail(e, "vi texture");
         }
         if ((s = check_launch(rs_tex_fill(sinogram, sinogram_dtype, g.nu, g.nv, g.np, ctx->vtex, st), "vi texture fill")) !=
@@ -507,6 +541,7 @@ tomo_status tomo_backproject(tomo_context* ctx, tomo_backprojector kind, const v
             pitch = vi_rows_pitch(g.nu);
             if (alloc_once(ctx, (void**)&ctx->rows, ctx->nsino_rows() * sizeof(float), false) != TOMO_OK) cudaGetLastError();
             rows = ctx->rows;
+            if (rows && !ctx->rows_held) ctx->rows_held = capturing(st);
             if (rows && (s = check_launch(launch_sino_rows(sinogram, sinogram_dtype, ctx->rows, g.nu, g.nv, g.np, (int)pitch, st),
                                           "sinogram rows")) != TOMO_OK)
                 return s;
@@ -688,7 +723,7 @@ tomo_status tomo_solver_create(tomo_context* ctx, const tomo_gradient_params* pr
     sv->log_cap = prm->gradient_iteration_nb > 0 ? prm->gradient_iteration_nb : 1;
     const size_t es = dtype_size(prm->storage);
     auto alloc = [&](void** p, size_t bytes, bool zero) -> bool {
-        return alloc_once(ctx, p, bytes, zero) == TOMO_OK;
+        return ensure(ctx, p, bytes, zero) == TOMO_OK;
     };
     bool ok = alloc(&sv->vpad, rs_input_elems(sv->rs_layout, ctx->hg.nx, ctx->hg.ny, ctx->hg.nz) * es, true) && alloc(&sv->spad, std::max(ctx->nsino_pad(), ctx->nsino_rows()) * sizeof(float), true) &&
               alloc((void**)&sv->dJ, ctx->nvox() * sizeof(float), false) &&
@@ -711,9 +746,10 @@ tomo_status tomo_solver_create(tomo_context* ctx, const tomo_gradient_params* pr
         ok = alloc((void**)&sv->partials, sv->npartials * sizeof(double), false);
     }
     if (ok && sv->rs_layout == RS_LAYOUT_MARCH)
-        ok = rs_march_tex_create(ctx->hg.nx, ctx->hg.ny, ctx->hg.nz, &sv->tex) == cudaSuccess;
+        ok = ensure_texture(ctx, [&] { return rs_march_tex_create(ctx->hg.nx, ctx->hg.ny, ctx->hg.nz, &sv->tex); }) == cudaSuccess;
     if (ok && vi_texture(ctx))
-        ok = rs_tex_create(ctx->hg.nu, ctx->hg.nv, ctx->hg.np, TOMO_F32, &sv->vtex, true) == cudaSuccess;
+        ok = ensure_texture(ctx, [&] { return rs_tex_create(ctx->hg.nu, ctx->hg.nv, ctx->hg.np, TOMO_F32, &sv->vtex, true); }) ==
+             cudaSuccess;
     if (ok) sv->vi_tma = !sv->vtex.tex && vi_staged(ctx);
     // last, and given back when a later allocation needs the room (ensure)
     if (ok && staged &&
@@ -839,6 +875,7 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
     if (!siddon && sv->rs_layout == RS_LAYOUT_TEX && !sv->stage.rows && !sv->tex.tex &&
         (s = solver_texture(sv)) != TOMO_OK)
         return s;
+    if (sv->stage.rows && !sv->stage_held) sv->stage_held = capturing(st);
     const size_t nparts = siddon           ? siddon_grid_blocks(g)
                           : sv->stage.rows ? rs_stage_grid_blocks(g)
                                            : rs_grid_blocks(sv->rs_layout, g);
