@@ -197,3 +197,18 @@ def test_copies_of_many_contexts_threads_and_streams(tomo):
 
     with cf.ThreadPoolExecutor(4) as ex:
         assert list(ex.map(work, range(4))) == [12] * 4
+
+
+@pytest.mark.parametrize("kind", ["VI", "VI_UM", "FDK"])
+@pytest.mark.parametrize("offset", [0, 4, 1000])
+def test_backprojection_over_its_sinogram(tomo, kind, offset):
+    """The volume may lie over the sinogram that it comes from: the same values."""
+    cfg = _cfg(tomo, 48, 48, 48, 48, 48, 48, 2.0)
+    n = 48 ** 3
+    buf = torch.empty(n + offset, device="cuda")
+    sino, vol = buf[:n].view(48, 48, 48), buf[offset:].view(48, 48, 48)
+    src = torch.rand(48, 48, 48, device="cuda")
+    with tomo.Context(cfg) as ctx:
+        ref = ctx.backproject(kind, src)
+        sino.copy_(src)
+        assert torch.equal(ctx.backproject(kind, sino, out=vol), ref)

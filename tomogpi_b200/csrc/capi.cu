@@ -533,11 +533,15 @@ tomo_status tomo_backproject(tomo_context* ctx, tomo_backprojector kind, const v
                             "vi_back_tex_kernel");
     }
     if ((kind == TOMO_BACK_VI || kind == TOMO_BACK_VI_UM || kind == TOMO_BACK_FDK) && vi_staged(ctx)) {
-        // the caller's FP32 rows where a tensor map can describe them, else a copy (one without
-        // memory for the copy takes the padded form, whose 16-bit copy is half the size)
+        // the caller's FP32 rows where a tensor map can describe them and the volume does not lie
+        // over them, else a copy (one without memory for the copy takes the padded form, whose
+        // 16-bit copy is half the size)
         const float* rows = (const float*)sinogram;
         long pitch = g.nu;
-        if (sinogram_dtype != TOMO_F32 || !vi_tma_supported(sinogram, g.nu)) {
+        const uintptr_t s0 = (uintptr_t)sinogram, v0 = (uintptr_t)volume;
+        const bool overlap = s0 < v0 + ctx->nvox() * dtype_size(volume_dtype) &&
+                             v0 < s0 + ctx->nsino() * dtype_size(sinogram_dtype);
+        if (sinogram_dtype != TOMO_F32 || overlap || !vi_tma_supported(sinogram, g.nu)) {
             pitch = vi_rows_pitch(g.nu);
             if (alloc_once(ctx, (void**)&ctx->rows, ctx->nsino_rows() * sizeof(float), false) != TOMO_OK) cudaGetLastError();
             rows = ctx->rows;
