@@ -202,12 +202,13 @@ def test_copies_of_many_contexts_threads_and_streams(tomo):
 @pytest.mark.parametrize("kind", ["VI", "VI_UM", "FDK"])
 @pytest.mark.parametrize("offset", [0, 4, 1000])
 def test_backprojection_over_its_sinogram(tomo, kind, offset):
-    """The volume may lie over the sinogram that it comes from: the same values."""
-    cfg = _cfg(tomo, 48, 48, 48, 48, 48, 48, 2.0)
-    n = 48 ** 3
-    buf = torch.empty(n + offset, device="cuda")
-    sino, vol = buf[:n].view(48, 48, 48), buf[offset:].view(48, 48, 48)
-    src = torch.rand(48, 48, 48, device="cuda")
+    """The volume may lie over the sinogram that it comes from: the same values. 1000 blocks, so the
+    later ones read what the first have written unless there is a copy."""
+    n = 160
+    cfg = _cfg(tomo, n, n, n, n, n, n, 2.0)
+    buf = torch.empty(n ** 3 + offset, device="cuda")
+    sino, vol = buf[:n ** 3].view(n, n, n), buf[offset:].view(n, n, n)
+    src = torch.rand(n, n, n, device="cuda")
     with tomo.Context(cfg) as ctx:
         ref = ctx.backproject(kind, src)
         sino.copy_(src)

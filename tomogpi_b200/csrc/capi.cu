@@ -162,6 +162,13 @@ bool capturing(cudaStream_t st) {
     return c != cudaStreamCaptureStatusNone;
 }
 
+// Lets the calling thread allocate while a stream is captured (the allocation is not captured).
+struct CaptureRelaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Makes room for another buffer: frees what the context's projections and backprojections can do
 // without (their staged copies, for the texture, half the size in FP32; their rows, for the padded
 // copy), unless a captured launch reads it. Whether anything was freed.
@@ -543,6 +550,7 @@ tomo_status tomo_backproject(tomo_context* ctx, tomo_backprojector kind, const v
                              v0 < s0 + ctx->nsino() * dtype_size(sinogram_dtype);
         if (sinogram_dtype != TOMO_F32 || overlap || !vi_tma_supported(sinogram, g.nu)) {
             pitch = vi_rows_pitch(g.nu);
+            const CaptureRelaxed relaxed;  // whether there is a copy depends on the sinogram's address
             if (alloc_once(ctx, (void**)&ctx->rows, ctx->nsino_rows() * sizeof(float), false) != TOMO_OK) cudaGetLastError();
             rows = ctx->rows;
             if (rows && !ctx->rows_held) ctx->rows_held = capturing(st);
