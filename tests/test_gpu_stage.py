@@ -99,8 +99,7 @@ VI = [(64, 64, 64, 64, 64, 9, 2.0), (128, 128, 128, 130, 126, 5, 2.0), (160, 157
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("spec", VI, ids=lambda s: "x".join(map(str, s)))
 def test_staged_backprojection_equals_padded(tomo, spec, dtype):
-    """VI and its UM variant: bit-identical to the padded copy's kernel (32 slices per thread).
-    FDK: the weights' reciprocal square root is within 2 ulp, so 1e-6 of the padded kernel."""
+    """VI, its UM variant and FDK: bit-identical to the padded copy's kernel (32 slices per thread)."""
     cfg = _cfg(tomo, *spec)
     sino = torch.from_numpy(np.random.default_rng(5).random(cfg.sinogram_shape, dtype=np.float32)).cuda().to(dtype)
     with tomo.Context(cfg) as ctx:
@@ -108,11 +107,7 @@ def test_staged_backprojection_equals_padded(tomo, spec, dtype):
         ctx.set_tuning(vi_zc=2)
         for k, v in got.items():
             ref = ctx.backproject(k, sino, dtype=torch.float32)
-            assert float(ref.abs().max()) > 0
-            if k == "FDK":
-                assert float(torch.linalg.vector_norm((v - ref).double()) / torch.linalg.vector_norm(ref.double())) <= 1e-6
-            else:
-                assert torch.equal(v, ref), k
+            assert float(ref.abs().max()) > 0 and torch.equal(v, ref), k
         torch.cuda.synchronize()
         assert ctx.errors() == 0
 

@@ -45,13 +45,6 @@ __device__ __forceinline__ bool vt_window(const DevGeom& g, int p, int x0, int x
     return (int)uhi - u0 < VT_BOX_U && (int)vhi - v0 < box_v;
 }
 
-// 1 / sqrt(x) within 2 ulp, for normal positive x (here at least betaC).
-__device__ __forceinline__ float vi_rsqrt(float x) {
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
 // The tensor map of a sinogram [P][nv][pitch] for NS slices per thread.
 bool vi_tma_encode(const float* sino, int nu, int nv, int np, long pitch, int ns, CUtensorMap* map);
 
@@ -180,13 +173,7 @@ __device__ __forceinline__ bool vi_tma_tile(const DevGeom& g, const CUtensorMap*
             for (int k = 0; k < skip; ++k) {  // the rows of the chunk's earlier slices (:410)
                 vn = fadd(vn, A);
             }
-        float fnum = 0.f, q0 = 0.f;
-        if (FDK) {  // alphaC (FDD/du) / denum^2 and betaC + u'^2 (FDK3D_kernel_16reg.cuh:77-84)
-            const float denum = fadd(fadd(fmul(fmul(xn, __ldg(g.alpha + p)), g.dx), fmul(fmul(yn, __ldg(g.beta + p)), g.dx)),
-                                     g.fod);
-            fnum = fdiv(fmul(g.fdk_alpha, g.fdd_du), fmul(denum, denum));
-            q0 = fmaf(up, up, g.fdk_beta);
-        }
+        const float2 fdk = FDK ? fdk_column(g, xn, yn, up, p) : make_float2(0.f, 0.f);
         if (!mbar_wait_warp(&sh.full[turn.s], turn.phase)) {
             if (lane == 0) atomicOr(err, ERR_TIMEOUT);
             alive = false;
@@ -214,10 +201,10 @@ __device__ __forceinline__ bool vi_tma_tile(const DevGeom& g, const CUtensorMap*
                 float2 t00, t10, t01, t11;
                 fetch((unsigned)__float_as_int(m.x), (unsigned)__float_as_int(m.y), t00, t10, t01, t11);
                 const float2 t = vi_bilerp2(t00, t10, t01, t11, aa, b);
-                if (FDK) {  // weight fnum / sqrt(betaC + u'^2 + v'^2), v' = v - vc
+                if (FDK) {  // fdk_weight of the two slices
                     const float2 vk = __fadd2_rn(vb, make_float2(-g.vc, -g.vc));
-                    const float2 q = __ffma2_rn(vk, vk, make_float2(q0, q0));
-                    const float2 w = __fmul2_rn(make_float2(fnum, fnum), make_float2(vi_rsqrt(q.x), vi_rsqrt(q.y)));
+                    const float2 q = __ffma2_rn(vk, vk, make_float2(fdk.y, fdk.y));
+                    const float2 w = __fmul2_rn(make_float2(fdk.x, fdk.x), make_float2(vi_rsqrt(q.x), vi_rsqrt(q.y)));
                     acc[k >> 1] = __ffma2_rn(w, t, acc[k >> 1]);
                 } else {
                     acc[k >> 1] = __fadd2_rn(acc[k >> 1], t);
