@@ -150,6 +150,13 @@ tomo_status tomo_context_set_tuning(tomo_context* ctx, const tomo_tuning* in);
    choice, or the cells where the texture's layer limit rules it out). */
 tomo_status tomo_context_rs_layout(const tomo_context* ctx, tomo_dtype dtype, int32_t* layout);
 
+/* Whether layout 2 of this context's projections, and of solvers created on it afterwards, is
+   staged in shared memory: 0 never (the texture's gathers, as a batch runs them), 1 where the
+   windows fit and that is the faster (default), 2 wherever they fit. */
+tomo_status tomo_context_set_staging(tomo_context* ctx, int32_t mode);
+/* Whether a projection of a volume of this type is staged (now). */
+tomo_status tomo_context_rs_staged(const tomo_context* ctx, tomo_dtype dtype, int32_t* staged);
+
 /* Projector<V,S,T>::doProjection(S* estimatedSinogram, V* volume)
    (src/TomoGPI_lib/inc/Projector.cuh:118): sinogram := H volume (overwrite).
    Device pointers. */

@@ -125,3 +125,47 @@ def test_autotuner_picks_and_caches(tmp_path, monkeypatch):
     assert set(r["trials"]) == {"rs_tex", "rs_hybrid", "rs_march", "rs_cell8", "rs_plain", "vi_zc1", "vi_zc2",
                                 "vi_zc4", "vi_tma"}
     assert (tmp_path / "tune.json").exists() and at.tune(cfg, "f32") == r
+
+
+@pytest.mark.parametrize("storage,n,views", [("bf16", 128, 48), ("bf16", 64, 48), ("f32", 64, 48)])
+def test_autotuner_times_what_runs(tmp_path, monkeypatch, storage, n, views):
+    """The trials of the texture layout: staged as the whole job's projections are, whatever the
+    trial's view count, and once as a batch's queue runs it, gathers in blocks of 32 x 8 rays."""
+    import tomogpi_b200.autotune as at
+    from tomogpi_b200 import ConfigCT, Context
+
+    monkeypatch.setattr(at, "_CACHE", tmp_path / "tune.json")
+    monkeypatch.setattr(at, "_mem", None)
+    seen = []
+    project = Context.project
+
+    def spy(self, kind, volume, **kw):
+        if self.tuning["rs_layout"] == "tex":
+            seen.append((self.views[1], self.tuning["rs_tile_u"], self.rs_staged(volume.dtype)))
+        return project(self, kind, volume, **kw)
+
+    monkeypatch.setattr(Context, "project", spy)
+    cfg = ConfigCT.cone_beam(n, views)
+    dt = {"f32": torch.float32, "bf16": torch.bfloat16}[storage]
+    with Context(cfg) as job:
+        staged = job.rs_staged(dt)
+    assert staged == (storage == "f32" or n == 128)
+    r = at.tune(cfg, storage, trial_views=24)
+    assert r["batch_layout"] in ("tex", "cell8", "plain")
+    assert set(seen) == {(v, 32, s) for v in (24, 48) for s in {staged, False}}
+
+
+def test_projection_staged_or_not_on_request():
+    """set_staging chooses between the staged copies and the texture's gathers; same values."""
+    from tomogpi_b200 import ConfigCT, Context
+
+    cfg = ConfigCT.cone_beam(40, 12)
+    vol = torch.rand(cfg.volume_shape, device="cuda")
+    out = {}
+    with Context(cfg) as ctx:
+        for dt in (torch.float32, torch.float16):
+            for mode, want in (("auto", dt == torch.float32), ("never", False), ("fits", True)):
+                ctx.set_staging(mode)
+                assert ctx.rs_staged(dt) == want
+                out[dt, mode] = ctx.project("RS", vol.to(dt), dtype=torch.float32)
+            assert torch.equal(out[dt, "auto"], out[dt, "never"]) and torch.equal(out[dt, "auto"], out[dt, "fits"])

@@ -76,6 +76,8 @@ SIGNATURES = {
     "tomo_context_get_tuning": (ctypes.c_int, [_vp, ctypes.POINTER(TomoTuning)]),
     "tomo_context_set_tuning": (ctypes.c_int, [_vp, ctypes.POINTER(TomoTuning)]),
     "tomo_context_test_stall": (ctypes.c_int, [_vp, ctypes.c_int]),
+    "tomo_context_set_staging": (ctypes.c_int, [_vp, _i32]),
+    "tomo_context_rs_staged": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.POINTER(_i32)]),
     "tomo_context_test_deny": (ctypes.c_int, [_vp, _i32, _i32]),
     "tomo_context_rs_layout": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.POINTER(_i32)]),
     "tomo_project": (ctypes.c_int, [_vp, ctypes.c_int, _vp, ctypes.c_int, _vp, ctypes.c_int, _vp]),

@@ -3,11 +3,11 @@ candidates on the device, and cache the choice.
 
 Candidates: RS layout in {tex, hybrid, cell8, plain, march}; VI slices per thread in
 {16, 32, 64} (vi_zc 1, 2, 4; 16 staged in shared memory by TMA, the others from the padded
-sinogram), and the staged form by name (vi_layout "tma"). "tex" is staged too where the
-geometry allows it; the batch's queue gathers from the texture, so its layout is picked with a
-trial of that form ("batch_layout"). The trials run the first k and 2k views of the job's own
-geometry, with CUDA-event timing after a warm-up, and are extrapolated to the job's view
-count. Results are cached in JSON (``$TOMOGPI_B200_TUNE_CACHE`` or
+sinogram), and the staged form by name (vi_layout "tma", the same kernel as vi_zc 1). "tex" is
+staged in the trials where the whole job's projections are; the batch's queue gathers from the
+texture in 32 x 8 blocks, so its layout is picked with a trial of just that ("batch_layout").
+The trials run the first k and 2k views of the job's own geometry, with CUDA-event timing after
+a warm-up, and are extrapolated to the job's view count. Results are cached in JSON (``$TOMOGPI_B200_TUNE_CACHE`` or
 ``~/.cache/tomogpi_b200/autotune.json``) keyed by the GPU name and the size class.
 """
 from __future__ import annotations
@@ -46,7 +46,7 @@ def _save():
 
 
 def size_key(cfg: ConfigCT, storage: str, gpu: str) -> str:
-    return (f"v4|{gpu}|{cfg.x_volume_pixel_nb}x{cfg.y_volume_pixel_nb}x{cfg.z_volume_pixel_nb}|"
+    return (f"v5|{gpu}|{cfg.x_volume_pixel_nb}x{cfg.y_volume_pixel_nb}x{cfg.z_volume_pixel_nb}|"
             f"{cfg.u_detector_pixel_nb}x{cfg.v_detector_pixel_nb}|{storage}")
 
 
@@ -60,9 +60,8 @@ def first_views(cfg: ConfigCT, k: int) -> ConfigCT:
 
 def pick(trials: dict) -> dict:
     """Fastest RS layout and VI form from {'rs_<layout>': ms, 'vi_zc<k>': ms, 'vi_tma': ms}:
-    the TMA form when it beats every padded chunking (its chunking is 16 slices), else the
-    fastest chunking; "vi_zc" is always a padded chunking (the batched kernels read the
-    padded residual)."""
+    the TMA form by name when it beats every chunking (its chunking is 16 slices), else the fastest
+    chunking; "vi_zc" is always the fastest of the chunkings, which is what a batch takes."""
     rs = {k[3:]: v for k, v in trials.items() if k.startswith("rs_")}
     vi = {int(k[5:]): v for k, v in trials.items() if k.startswith("vi_zc")}
     zc = min(vi, key=vi.get)
@@ -118,18 +117,20 @@ def tune(cfg: ConfigCT, storage: str = "f32", device: int = 0, trial_views: int 
     layouts = ("tex", "hybrid", "cell8") if big else ("tex", "hybrid", "cell8", "plain")
     if storage == "f32":  # MARCH is an FP32 layout (16-bit storage runs it as TEX)
         layouts += ("march",)
+    with Context(cfg, device=device) as job:  # staging depends on the view count too (16-bit volumes)
+        staged = job.rs_staged(tdt)
     for views in sorted({k, min(2 * k, P)}):
         sub = first_views(cfg, views)
         with Context(sub, device=device) as ctx:
             vol = torch.rand(sub.volume_shape, device=dev).to(tdt)
             sino = torch.empty(sub.sinogram_shape, device=dev, dtype=tdt)
+            ctx.set_staging("fits" if staged else "never")
             for lay in layouts:
                 ctx.set_tuning(rs_layout=lay)
                 raw[(f"rs_{lay}", views)] = _time(lambda: ctx.project("RS", vol, out=sino), reps=2)
-            # 128 rays wide, a block's windows fit no stage: the texture's gathers
-            ctx.set_tuning(rs_layout="tex", rs_tile_u=128)
+            ctx.set_staging("never")
+            ctx.set_tuning(rs_layout="tex")
             raw[("gather", views)] = _time(lambda: ctx.project("RS", vol, out=sino), reps=2)
-            ctx.set_tuning(rs_tile_u=32)
             res = torch.rand(sub.sinogram_shape, device=dev)
             dj = torch.empty(sub.volume_shape, device=dev)
             for zc in vi_zcs:

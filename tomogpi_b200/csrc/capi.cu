@@ -56,6 +56,7 @@ struct tomo_context {
     RsTexture tex;                       // TEX layout: layered array of the volume's type
     RsStage stage;                       // TEX layout, staged: the volume's copies
     bool stage_denied = false;           // no memory for them: the texture instead
+    int staging = 1;                     // 0 the texture only, 1 the copies where they are faster, 2 where they fit
     bool stage_held = false, rows_held = false;  // a captured launch reads them: kept as long as the context
     RsTexture vtex;                      // VI texture layout: layered array of the sinogram
     float* d_ramp = nullptr;             // ramp-filter taps for (ramp_over, ramp_cut)
@@ -283,6 +284,10 @@ int effective_layout(int requested, tomo_dtype vdt, int nx, int ny, int nz) {
     return requested;
 }
 
+bool rs_staged(const tomo_context* ctx, tomo_dtype vdt) {
+    return ctx->staging == 2 ? rs_stage_fits(ctx->g) : ctx->staging == 1 && rs_stage_supported(ctx->g, vdt);
+}
+
 // The context's texture for a volume of type vdt (MARCH: its even faces), created or replaced
 // where it is of another kind, filled from the volume.
 tomo_status context_texture(tomo_context* ctx, bool march, const void* vol, tomo_dtype vdt, cudaStream_t st) {
@@ -308,7 +313,7 @@ tomo_status project_into(tomo_context* ctx, tomo_projector kind, const void* vol
     const DevGeom& g = ctx->g;
     if (kind == TOMO_PROJ_RS || kind == TOMO_PROJ_RS_UM) {
         const int layout = effective_layout(ctx->tuning.rs_layout, vdt, g.nx, g.ny, g.nz);
-        bool staged = layout == RS_LAYOUT_TEX && !ctx->stage_denied && rs_stage_supported(g, vdt);
+        bool staged = layout == RS_LAYOUT_TEX && !ctx->stage_denied && rs_staged(ctx, vdt);
         if (staged && ctx->stage.rows && ctx->stage.dt != vdt) {  // copies of another type
             if (ctx->stage_held) {
                 staged = false;
@@ -470,6 +475,20 @@ tomo_status tomo_context_get_tuning(const tomo_context* ctx, tomo_tuning* out) {
 tomo_status tomo_context_rs_layout(const tomo_context* ctx, tomo_dtype dtype, int32_t* layout) {
     TOMO_CHECK_ARG(ctx && layout && valid_dtype(dtype), "tomo_context_rs_layout: bad argument");
     *layout = effective_layout(ctx->tuning.rs_layout, dtype, ctx->hg.nx, ctx->hg.ny, ctx->hg.nz);
+    return TOMO_OK;
+}
+
+tomo_status tomo_context_set_staging(tomo_context* ctx, int32_t mode) {
+    TOMO_CHECK_ARG(ctx && mode >= 0 && mode <= 2, "tomo_context_set_staging: mode must be 0, 1 or 2");
+    ctx->staging = mode;
+    return TOMO_OK;
+}
+
+tomo_status tomo_context_rs_staged(const tomo_context* ctx, tomo_dtype dtype, int32_t* staged) {
+    TOMO_CHECK_ARG(ctx && staged && valid_dtype(dtype), "tomo_context_rs_staged: bad argument");
+    const HostGeom& h = ctx->hg;
+    *staged = effective_layout(ctx->tuning.rs_layout, dtype, h.nx, h.ny, h.nz) == RS_LAYOUT_TEX && !ctx->stage_denied &&
+              rs_staged(ctx, dtype);
     return TOMO_OK;
 }
 
@@ -745,7 +764,7 @@ tomo_status tomo_solver_create(tomo_context* ctx, const tomo_gradient_params* pr
     if (ok && prm->storage != TOMO_F32 && (prm->projector == TOMO_PROJ_SIDDON || prm->projector == TOMO_PROJ_SIDDON_REF))
         ok = alloc(&sv->vplain, ctx->nvox() * es, false);
     const bool rs = prm->projector == TOMO_PROJ_RS || prm->projector == TOMO_PROJ_RS_UM;
-    const bool staged = rs && sv->rs_layout == RS_LAYOUT_TEX && rs_stage_supported(ctx->g, prm->storage);
+    const bool staged = rs && sv->rs_layout == RS_LAYOUT_TEX && rs_staged(ctx, prm->storage);
     if (ok && !(staged && prm->storage == TOMO_F32) &&
         (sv->rs_layout == RS_LAYOUT_TEX || sv->rs_layout == RS_LAYOUT_HYBRID))
         ok = solver_texture(sv) == TOMO_OK;

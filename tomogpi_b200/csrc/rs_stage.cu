@@ -69,14 +69,18 @@ __global__ void __launch_bounds__(256) rs_stage_fill_kernel(const Ti* __restrict
 static int stage_slices(tomo_dtype dt, int nz) { return dt == TOMO_F32 ? nz : nz + 1; }
 static int pitch4(int n) { return (n + 3) & ~3; }
 
-bool rs_stage_supported(const DevGeom& g, tomo_dtype dt) {
+bool rs_stage_fits(const DevGeom& g) {
     if (!tma_encode_fn() || !g.view_order || std::max({g.nx, g.ny, g.nz}) > 4096) return false;
     // A tile's window at the volume's centre, worst over the view angles: a stage has to hold
     // four of its planes or more (at spacings of several voxels per pixel a staged word
     // serves less than one sample, and the gathers of the texture are faster).
     const float su = g.du * g.fod / (g.fdd * g.dx), sv = g.dv * g.fod / (g.fdd * g.dx);
     const float w = 1.42f * su * (float)rs_tile_u(g) * 1.2f + 12.0f, h = sv * (float)rs_tile_v(g) * 1.2f + 6.0f;
-    if (!(w <= 84.0f && h <= 32.0f && w * h * 4.0f <= (float)RSG_CAP)) return false;
+    return w <= 84.0f && h <= 32.0f && w * h * 4.0f <= (float)RSG_CAP;
+}
+
+bool rs_stage_supported(const DevGeom& g, tomo_dtype dt) {
+    if (!rs_stage_fits(g)) return false;
     if (dt == TOMO_F32) return true;
     // 16-bit volumes gain about a tenth of the projection for a second fill of 8 B a voxel: not
     // below 128^3 (BF16, 64^3, 60 views: 71 us against 61; 128^3, 128 views: 477 against 492),

@@ -25,6 +25,7 @@ PROJECTORS = {"RS": L.PROJ_RS, "RS_UM": L.PROJ_RS_UM, "SIDDON_REF": L.PROJ_SIDDO
 LAYOUTS = {"plain": L.RS_LAYOUT_PLAIN, "cell8": L.RS_LAYOUT_CELL8, "tex": L.RS_LAYOUT_TEX, "hybrid": L.RS_LAYOUT_HYBRID,
            "march": L.RS_LAYOUT_MARCH}
 LAYOUT_NAMES = {v: k for k, v in LAYOUTS.items()}
+STAGING = {"never": 0, "auto": 1, "fits": 2}
 VI_LAYOUTS = {"padded": 0, "tex": 1, "tma": 2}
 VI_LAYOUT_NAMES = {v: k for k, v in VI_LAYOUTS.items()}
 BACKPROJECTORS = {"VI": L.BACK_VI, "VI_UM": L.BACK_VI_UM, "RS_ADJOINT": L.BACK_RS_ADJOINT,
@@ -114,6 +115,18 @@ class Context:
         code = {torch.float32: L.F32, torch.bfloat16: L.BF16, torch.float16: L.F16}[dtype or torch.float32]
         L.call("tomo_context_rs_layout", self._h, code, ctypes.byref(out))
         return LAYOUT_NAMES[out.value]
+
+    def rs_staged(self, dtype=None) -> bool:
+        """Whether a projection of a volume of `dtype` is staged in shared memory (the "tex" layout)."""
+        out = ctypes.c_int32()
+        code = {torch.float32: L.F32, torch.bfloat16: L.BF16, torch.float16: L.F16}[dtype or torch.float32]
+        L.call("tomo_context_rs_staged", self._h, code, ctypes.byref(out))
+        return bool(out.value)
+
+    def set_staging(self, mode: str = "auto") -> None:
+        """When the "tex" layout is staged: "never" | "auto" (where that is the faster) | "fits" (wherever
+        the geometry allows it). Set before creating solvers on the context."""
+        L.call("tomo_context_set_staging", self._h, STAGING[mode])
 
     def set_tuning(self, rs_layout=None, vi_zc=None, vi_layout=None, rs_warp_u=None, rs_tile_u=None) -> None:
         """rs_layout: "tex" | "hybrid" | "march" | "cell8" | "plain"; vi_zc: 1 | 2 | 4; vi_layout: "tex" | "padded" | "tma";
