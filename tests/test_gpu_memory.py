@@ -28,6 +28,13 @@ def _cfg(tomo, n=40, views=12):
     return tomo.ConfigCT.cone_beam(n, views)
 
 
+def _context(tomo, cfg):
+    """A context that stages its projections wherever the geometry allows it."""
+    ctx = tomo.Context(cfg)
+    ctx.set_staging("fits")
+    return ctx
+
+
 def _volume(cfg, seed=1):
     return torch.from_numpy(np.random.default_rng(seed).random(cfg.volume_shape, dtype=np.float32)).cuda()
 
@@ -41,18 +48,18 @@ def test_projection_without_room_for_the_copies(tomo):
     texture from then on. Bit-identical either way."""
     cfg = _cfg(tomo)
     vol = _volume(cfg)
-    with tomo.Context(cfg) as ctx:
+    with _context(tomo, cfg) as ctx:
         ref = ctx.project("RS", vol)
-    with tomo.Context(cfg) as ctx:
+    with _context(tomo, cfg) as ctx:
         _deny(ctx, 1, 1)  # after the projector's input buffer
         assert torch.equal(ctx.project("RS", vol), ref)
         assert torch.equal(ctx.project("RS", vol), ref)
-    with tomo.Context(cfg) as ctx:
+    with _context(tomo, cfg) as ctx:
         ctx.project("RS", vol)
         _deny(ctx, 0, 1)  # the host form's volume
         assert np.array_equal(ctx.project_host("RS", vol.cpu().numpy()), ref.cpu().numpy())
         assert torch.equal(ctx.project("RS", vol), ref)
-    with tomo.Context(cfg) as ctx:
+    with _context(tomo, cfg) as ctx:
         _deny(ctx, 1, 2)  # neither the copies nor the texture
         with pytest.raises(RuntimeError, match="NO_MEMORY"):
             ctx.project("RS", vol)
@@ -65,9 +72,9 @@ def test_backprojection_without_room_for_the_rows(tomo, dtype):
     the next call runs."""
     cfg = _cfg(tomo).replace(u_detector_pixel_nb=42)
     s = _sino(cfg).to(dtype)
-    with tomo.Context(cfg) as ctx:
+    with _context(tomo, cfg) as ctx:
         ref = ctx.backproject("VI", s, dtype=torch.float32)
-    with tomo.Context(cfg) as ctx:
+    with _context(tomo, cfg) as ctx:
         _deny(ctx, 0, 2)
         with pytest.raises(RuntimeError, match="NO_MEMORY"):
             ctx.backproject("VI", s, dtype=torch.float32)
@@ -86,7 +93,7 @@ def test_solver_creation_with_one_failed_allocation(tomo, storage):
     cfg = _cfg(tomo)
     s = _sino(cfg)
     par = _params(tomo, storage=storage, real_f32=True)
-    with tomo.Context(cfg) as ctx:
+    with _context(tomo, cfg) as ctx:
         ref = tomo.Solver(ctx, par).iterate(_volume(cfg), s).cpu().numpy()
         made = 0
         for skip in range(14):
@@ -144,7 +151,7 @@ def test_solver_whose_copies_gave_way(tomo, step, fails):
         insist(lambda: solver.iterate(vol, s))
         return vol.cpu().numpy(), tries
 
-    with tomo.Context(cfg) as ctx:
+    with _context(tomo, cfg) as ctx:
         ref, none = run(tomo.Solver(ctx, _params(tomo)), 0)
         got, tries = run(tomo.Solver(ctx, _params(tomo)), fails)
         _deny(ctx, 0, 0)
@@ -164,7 +171,7 @@ def test_captured_launches_keep_their_buffers(tomo):
     buffer or to a volume of another type: the replay is exact after either."""
     cfg = _cfg(tomo, n=128, views=45).replace(u_detector_pixel_nb=126)
     vol, s = _volume(cfg), _sino(cfg).to(torch.bfloat16)
-    with tomo.Context(cfg) as ctx:
+    with _context(tomo, cfg) as ctx:
         fwd, back = ctx.project("RS", vol), ctx.backproject("VI", s, dtype=torch.float32)
         ref, bref = fwd.clone(), back.clone()
         g = _captured(lambda: (ctx.project("RS", vol, out=fwd), ctx.backproject("VI", s, out=back)))
@@ -185,7 +192,7 @@ def test_captured_iterations_keep_the_solvers_copies(tomo):
     """The same for the copies that a solver's captured iterations read."""
     cfg = _cfg(tomo)
     s = _sino(cfg)
-    with tomo.Context(cfg) as ctx:
+    with _context(tomo, cfg) as ctx:
         sv = tomo.Solver(ctx, _params(tomo))
         vol = _volume(cfg)
         ref = sv.iterate(vol, s).clone()
@@ -205,9 +212,9 @@ def test_copies_give_way_to_a_new_solver(tomo):
     """A solver that finds no room takes that of the context's copies and rows."""
     cfg = _cfg(tomo).replace(u_detector_pixel_nb=42)
     vol, s = _volume(cfg), _sino(cfg)
-    with tomo.Context(cfg) as ctx:
+    with _context(tomo, cfg) as ctx:
         ref = tomo.Solver(ctx, _params(tomo)).iterate(vol.clone(), s)
-    with tomo.Context(cfg) as ctx:
+    with _context(tomo, cfg) as ctx:
         fwd, back = ctx.project("RS", vol), ctx.backproject("VI", s)
         _deny(ctx, 1, 1)
         assert rel_l2(tomo.Solver(ctx, _params(tomo)).iterate(vol.clone(), s).cpu().numpy(), ref.cpu().numpy()) <= 1e-6
@@ -220,7 +227,7 @@ def test_capture_with_a_sinogram_that_needs_rows(tomo):
     cfg = _cfg(tomo)
     s = _sino(cfg)
     odd = torch.empty(s.numel() + 1, device="cuda")[1:].view(s.shape).copy_(s)
-    with tomo.Context(cfg) as ctx:
+    with _context(tomo, cfg) as ctx:
         back = ctx.backproject("VI", s)
         ref = back.clone()
         back.zero_()

@@ -127,8 +127,8 @@ def test_autotuner_picks_and_caches(tmp_path, monkeypatch):
     assert (tmp_path / "tune.json").exists() and at.tune(cfg, "f32") == r
 
 
-@pytest.mark.parametrize("storage,n,views", [("bf16", 128, 48), ("bf16", 64, 48), ("f32", 64, 48)])
-def test_autotuner_times_what_runs(tmp_path, monkeypatch, storage, n, views):
+@pytest.mark.parametrize("storage,n,views,det", [("bf16", 128, 48, 256), ("bf16", 64, 48, 64), ("f32", 64, 48, 64)])
+def test_autotuner_times_what_runs(tmp_path, monkeypatch, storage, n, views, det):
     """The trials of the texture layout: staged as the whole job's projections are, whatever the
     trial's view count, and once as a batch's queue runs it, gathers in blocks of 32 x 8 rays."""
     import tomogpi_b200.autotune as at
@@ -145,7 +145,7 @@ def test_autotuner_times_what_runs(tmp_path, monkeypatch, storage, n, views):
         return project(self, kind, volume, **kw)
 
     monkeypatch.setattr(Context, "project", spy)
-    cfg = ConfigCT.cone_beam(n, views)
+    cfg = ConfigCT.cone_beam(n, views, det=det, pitch=2.0 * n / det)
     dt = {"f32": torch.float32, "bf16": torch.bfloat16}[storage]
     with Context(cfg) as job:
         staged = job.rs_staged(dt)
@@ -159,7 +159,7 @@ def test_projection_staged_or_not_on_request():
     """set_staging chooses between the staged copies and the texture's gathers; same values."""
     from tomogpi_b200 import ConfigCT, Context
 
-    cfg = ConfigCT.cone_beam(40, 12)
+    cfg = ConfigCT.cone_beam(64, 60)
     vol = torch.rand(cfg.volume_shape, device="cuda")
     out = {}
     with Context(cfg) as ctx:

@@ -1,5 +1,5 @@
-"""The forms staged in shared memory by TMA that the default tuning runs: the RS projector of
-FP32 volumes (csrc/rs_stage.cuh) and the VI and FDK backprojectors (csrc/vi_tma.cu), against
+"""The forms staged in shared memory by TMA that the default tuning runs: the RS projector
+(csrc/rs_stage.cuh; where the geometry allows it, as set_staging("fits") asks for here) and the VI and FDK backprojectors (csrc/vi_tma.cu), against
 the forms that read global memory."""
 import numpy as np
 import pytest
@@ -39,6 +39,7 @@ def test_staged_projection_equals_padded(tomo, spec, kind):
     cfg = _cfg(tomo, *spec)
     vol = torch.from_numpy(np.random.default_rng(3).random(cfg.volume_shape, dtype=np.float32) + 0.25).cuda()
     with tomo.Context(cfg) as ctx:
+        ctx.set_staging("fits")
         got = ctx.project(kind, vol)
         half = ctx.project(kind, vol, dtype=torch.bfloat16)
         ctx.set_tuning(rs_layout="plain")
@@ -64,7 +65,9 @@ def test_half_staged_projection_equals_cells(tomo, spec, storage):
     out = {}
     for lay in ("tex", "cell8"):
         with tomo.Context(cfg) as ctx:
+            ctx.set_staging("fits")
             ctx.set_tuning(rs_layout=lay)
+            assert ctx.rs_staged(storage) == (lay == "tex")
             out[lay] = [ctx.project(k, vol.to(storage), dtype=torch.float32) for k in ("RS", "RS_UM")]
             f = vol.clone()
             tomo.Solver(ctx, par).iterate(f, real)
@@ -83,6 +86,7 @@ def test_staged_projection_launch_shapes(tomo, tile):
     cfg = _cfg(tomo, 70, 70, 50, 150, 61, 8, 1.0)
     vol = torch.rand(cfg.volume_shape, device="cuda")
     with tomo.Context(cfg) as ctx:
+        ctx.set_staging("fits")
         ctx.set_tuning(rs_warp_u=tile[0], rs_tile_u=tile[1])
         got = ctx.project("RS", vol)
         ctx.set_tuning(rs_layout="plain")
@@ -120,6 +124,7 @@ def test_staged_copies_remade_at_the_same_address(tomo):
         cfg = _cfg(tomo, n, n, n, n, n, views, 2.0)
         vol = torch.rand(cfg.volume_shape, device="cuda")
         with tomo.Context(cfg) as ctx, tomo.Context(cfg) as plain:
+            ctx.set_staging("fits")
             plain.set_tuning(rs_layout="cell8")
             for dt in (torch.float32, torch.bfloat16, torch.float32, torch.float16, torch.bfloat16):
                 v = vol.to(dt)
@@ -136,6 +141,7 @@ def test_closed_contexts_give_their_copies_back(tomo, dtype, n, views):
     free = []
     for _ in range(6):
         with tomo.Context(cfg) as ctx:
+            ctx.set_staging("fits")
             ctx.project("RS", vol, out=out)
             torch.cuda.synchronize()
         free.append(torch.cuda.mem_get_info()[0])
@@ -153,6 +159,7 @@ def test_staged_projection_bounded_wait_reports_timeout(tomo, dtype, n, views):
     cfg = _cfg(tomo, n, n, n, 128 if n == 128 else 16, 128 if n == 128 else 8, views, 2.0)
     vol = torch.rand(cfg.volume_shape, device="cuda").to(dtype)
     with tomo.Context(cfg, views=(0, 1) if n == 16 else None) as ctx:
+        ctx.set_staging("fits")
         ref = ctx.project("RS", vol)
         torch.cuda.synchronize()
         assert ctx.errors(clear=True) == 0
@@ -185,6 +192,7 @@ def test_copies_of_many_contexts_threads_and_streams(tomo):
             for i in range(12):
                 j = (k + i) % len(cfgs)
                 with tomo.Context(cfgs[j]) as ctx:
+                    ctx.set_staging("fits")
                     out = ctx.project("RS", vols[j])
                     st.synchronize()
                     good += int(torch.equal(out, refs[j]))
@@ -208,3 +216,27 @@ def test_backprojection_over_its_sinogram(tomo, kind, offset):
         ref = ctx.backproject(kind, src)
         sino.copy_(src)
         assert torch.equal(ctx.backproject(kind, sino, out=vol), ref)
+
+
+# (nx, ny, nz, nu, nv, views, pitch, mag[, fod]), FP32 staged?, 16-bit staged?
+RULE = [((256, 256, 256, 256, 256, 64, 1.6), True, True), ((64, 64, 64, 64, 64, 60, 2.0), True, False),
+        ((128, 128, 128, 256, 256, 60, 1.0), True, True), ((20, 20, 20, 20, 20, 60, 2.0), False, False),
+        ((33, 33, 500, 33, 500, 30, 2.0), False, False), ((160, 160, 160, 123, 123, 40, 2.6, 2.0, 120.0), False, False),
+        ((160, 160, 160, 133, 133, 60, 2.4), True, False), ((64, 64, 64, 20, 20, 9, 8.0), False, False)]
+
+
+@pytest.mark.parametrize("spec,f32,half", RULE, ids=lambda s: "x".join(map(str, s)) if isinstance(s, tuple) else str(s))
+def test_staged_where_it_is_faster(tomo, spec, f32, half):
+    """The rule takes what the measurements behind it say, for both types, whatever was projected
+    before; and the values do not depend on it (bit-identical to the padded layout)."""
+    cfg = _cfg(tomo, *spec)
+    vol = torch.rand(cfg.volume_shape, device="cuda")
+    with tomo.Context(cfg) as ctx, tomo.Context(cfg) as plain:
+        plain.set_tuning(rs_layout="plain")
+        for dt, want in ((torch.float32, f32), (torch.bfloat16, half), (torch.float16, half), (torch.float32, f32)):
+            assert ctx.rs_staged(dt) == want
+            v = vol.to(dt)
+            assert torch.equal(ctx.project("RS", v, dtype=torch.float32), plain.project("RS", v, dtype=torch.float32))
+        ctx.set_tuning(rs_warp_u=32, rs_tile_u=128)
+        ctx.set_tuning(rs_warp_u=8, rs_tile_u=32)
+        assert ctx.rs_staged(torch.float32) == f32

@@ -57,6 +57,7 @@ struct tomo_context {
     RsStage stage;                       // TEX layout, staged: the volume's copies
     bool stage_denied = false;           // no memory for them: the texture instead
     int staging = 1;                     // 0 the texture only, 1 the copies where they are faster, 2 where they fit
+    bool stage_fits[2] = {false, false}, stage_pays[2] = {false, false};  // FP32, 16-bit volumes: of this launch shape
     bool stage_held = false, rows_held = false;  // a captured launch reads them: kept as long as the context
     RsTexture vtex;                      // VI texture layout: layered array of the sinogram
     float* d_ramp = nullptr;             // ramp-filter taps for (ramp_over, ramp_cut)
@@ -285,7 +286,17 @@ int effective_layout(int requested, tomo_dtype vdt, int nx, int ny, int nz) {
 }
 
 bool rs_staged(const tomo_context* ctx, tomo_dtype vdt) {
-    return ctx->staging == 2 ? rs_stage_fits(ctx->g) : ctx->staging == 1 && rs_stage_supported(ctx->g, vdt);
+    const int k = vdt == TOMO_F32 ? 0 : 1;
+    return ctx->staging == 2 ? ctx->stage_fits[k] : ctx->staging == 1 && ctx->stage_pays[k];
+}
+// Once the geometry and the launch shape are known.
+void rate_staging(tomo_context* ctx) {
+    for (int k = 0; k < 2; ++k) {
+        const tomo_dtype dt = k ? TOMO_BF16 : TOMO_F32;
+        const RsStageFit f = rs_stage_fit(ctx->g, dt);
+        ctx->stage_fits[k] = f.fits;
+        ctx->stage_pays[k] = rs_stage_pays(f, ctx->g, dt);
+    }
 }
 
 // The context's texture for a volume of type vdt (MARCH: its even faces), created or replaced
@@ -424,6 +435,7 @@ tomo_status tomo_context_create_views(const tomo_config_ct* cfg, int device, int
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->host_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return fail(cuda_fail(e, "tomo_context_create"));
     fill_devgeom(h, ctx->d_alpha, ctx->d_beta, ctx->d_vi, ctx->g, ctx->d_order);
+    rate_staging(ctx);
     *out = ctx;
     return TOMO_OK;
 }
@@ -503,7 +515,9 @@ tomo_status tomo_context_set_tuning(tomo_context* ctx, const tomo_tuning* in) {
                    "64 or 128, rs_warp_u <= rs_tile_u");
     ctx->tuning = *in;
     if (ctx->tuning.vi_zc == 0) ctx->tuning.vi_zc = 1;
+    const int wl = ctx->g.rs_wlog, tl = ctx->g.rs_tlog;
     rs_shape_of(ctx->tuning, ctx->g);
+    if (ctx->g.rs_wlog != wl || ctx->g.rs_tlog != tl) rate_staging(ctx);
     return TOMO_OK;
 }
 

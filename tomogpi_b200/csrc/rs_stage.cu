@@ -2,6 +2,7 @@
 // kernel, the two volume copies that it reads and their tensor maps.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <mutex>
 #include <new>
 
@@ -69,24 +70,111 @@ __global__ void __launch_bounds__(256) rs_stage_fill_kernel(const Ti* __restrict
 static int stage_slices(tomo_dtype dt, int nz) { return dt == TOMO_F32 ? nz : nz + 1; }
 static int pitch4(int n) { return (n + 3) & ~3; }
 
-bool rs_stage_fits(const DevGeom& g) {
-    if (!tma_encode_fn() || !g.view_order || std::max({g.nx, g.ny, g.nz}) > 4096) return false;
-    // A tile's window at the volume's centre, worst over the view angles: a stage has to hold
-    // four of its planes or more (at spacings of several voxels per pixel a staged word
-    // serves less than one sample, and the gathers of the texture are faster).
-    const float su = g.du * g.fod / (g.fdd * g.dx), sv = g.dv * g.fod / (g.fdd * g.dx);
-    const float w = 1.42f * su * (float)rs_tile_u(g) * 1.2f + 12.0f, h = sv * (float)rs_tile_v(g) * 1.2f + 6.0f;
-    return w <= 84.0f && h <= 32.0f && w * h * 4.0f <= (float)RSG_CAP;
+// What the producer would stage (rsg_produce) for a few tiles, planes and directions of the
+// geometry: 27 tiles x 6 planes, about 10 us, once per geometry and launch shape.
+RsStageFit rs_stage_fit(const DevGeom& g, tomo_dtype dt) {
+    RsStageFit f;
+    if (!tma_encode_fn() || !g.view_order || std::max({g.nx, g.ny, g.nz}) > 4096) return f;
+    // a tile's window at the volume's centre, worst over the view angles: a stage holds four of its
+    // planes or more
+    const double su = g.du * g.fod / (g.fdd * g.dx), sv = g.dv * g.fod / (g.fdd * g.dx);
+    const double w0 = 1.42 * su * rs_tile_u(g) * 1.2 + 12.0, h0 = sv * rs_tile_v(g) * 1.2 + 6.0;
+    f.fits = w0 <= 84.0 && h0 <= 32.0 && w0 * h0 * 4.0 <= RSG_CAP;
+    if (!f.fits) return f;
+    const int tu = rs_tile_u(g), tv = rs_tile_v(g), nut = rs_tiles_u(g), nvt = rs_tiles_v(g);
+    const double edge = dt == TOMO_F32 ? 2.5 : 1.5;  // rows beside a window's span: FP32 slices / slice pairs
+    const double fod = g.fod / g.dx, fdd = g.fdd / g.dx, du = g.du / g.dx, dv = g.dv / g.dx;
+    double samples = 0, words = 0, missed = 0, length = 0;
+    int tiles = 0;
+    for (int d = 0; d < (g.nx == g.ny ? 3 : 6); ++d) {  // three directions of the first octant, and across it
+        const double phi = d < 3 ? 0.1 + 0.3 * d : M_PI / 2 - 0.1 - 0.3 * (d - 3), al = std::cos(phi), be = std::sin(phi);
+        for (int i = 0; i < 9; ++i) {
+            const int ut = (2 * (i % 3) + 1) * nut / 6, vt = (2 * (i / 3) + 1) * nvt / 6;
+            const int u0 = ut * tu, u1 = std::min(u0 + tu, g.nu) - 1, v0 = vt * tv, v1 = std::min(v0 + tv, g.nv) - 1;
+            // the axis that the tile's central ray runs along
+            const double um = 0.5 * (u0 + u1), cm = (um - g.uc) * du;
+            const bool xm = std::fabs(al * fdd - cm * be) >= std::fabs(be * fdd + cm * al);
+            const double nm = xm ? g.nx : g.ny, nt = xm ? g.ny : g.nx;
+            const double ms = (xm ? g.xc : g.yc) - fod * (xm ? al : be), ts = (xm ? g.yc : g.xc) - fod * (xm ? be : al);
+            // a ray's steps along and across it for detector column u
+            auto along = [&](double u) { const double c = (u - g.uc) * du; return xm ? al * fdd - c * be : be * fdd + c * al; };
+            auto across = [&](double u) { const double c = (u - g.uc) * du; return xm ? be * fdd + c * al : al * fdd - c * be; };
+            const double m = along(um), t = across(um), z = (0.5 * (v0 + v1) - g.vc) * dv;
+            double lo = 0, hi = nm - 1;  // planes that the central ray crosses inside the volume
+            const double c[2] = {ts, g.zc}, s[2] = {t / m, z / m}, n[2] = {nt - 1, (double)g.nz - 1};
+            for (int k = 0; k < 2; ++k) {
+                const double p0 = (0 - c[k]) / s[k], p1 = (n[k] - c[k]) / s[k];
+                if (std::fabs(s[k]) < 1e-9) continue;
+                lo = std::max(lo, ms + std::min(p0, p1));
+                hi = std::min(hi, ms + std::max(p0, p1));
+            }
+            if (!(hi - lo >= 1)) continue;
+            const double a0 = along(u0), a1 = along(u1);
+            const double steps = (hi - lo + 1) * std::sqrt(m * m + t * t + z * z) / std::fabs(m);
+            const double here = steps * (u1 - u0 + 1) * (v1 - v0 + 1);
+            samples += here;
+            length += steps;
+            ++tiles;
+            if (!(std::min(a0, a1) > 0.25 * fdd || std::max(a0, a1) < -0.25 * fdd)) {
+                missed += here;
+                continue;
+            }
+            const double st[2] = {across(u0) / a0, across(u1) / a1};
+            double zl = 1e30, zh = -1e30;
+            for (int k = 0; k < 4; ++k) {
+                const double q = ((k & 1 ? v1 : v0) - g.vc) * dv / (k & 2 ? a1 : a0);
+                zl = std::min(zl, q);
+                zh = std::max(zh, q);
+            }
+            const double sl[2] = {std::min(st[0], st[1]), zl}, sh[2] = {std::max(st[0], st[1]), zh};
+            for (int k = 0; k < 6; ++k) {
+                const double p = std::floor(lo + k * (hi - lo) / 5.0), weight = (k % 5 ? 0.2 : 0.1);
+                double best = 0;
+                for (int C = 1; C <= RSG_CMAX && C <= hi - lo + 1; ++C) {
+                    const double e0 = p - 0.5 * (C - 1) - 0.15 - ms, e1 = p + 0.5 * (C + 1) + 0.15 - ms;
+                    double span[2];
+                    for (int q = 0; q < 2; ++q)
+                        span[q] = std::max({e0 * sl[q], e0 * sh[q], e1 * sl[q], e1 * sh[q]}) -
+                                  std::min({e0 * sl[q], e0 * sh[q], e1 * sl[q], e1 * sh[q]}) + 0.2;
+                    int wi = 0, hj = 0;
+                    while (wi < RSG_WIDTHS && rsg_width(wi) < span[0] + 3.5) ++wi;
+                    while (hj < RSG_HEIGHTS && rsg_height(hj) < span[1] + edge) ++hj;
+                    const int wh = rsg_width(wi) * rsg_height(hj);
+                    if (wi == RSG_WIDTHS || hj == RSG_HEIGHTS || (C + 2) * ((wh + 31) & ~31) > RSG_CAP) break;
+                    best = (C + 2.0) * wh / C;  // words per plane
+                }
+                if (best > 0) words += weight * best * (hi - lo + 1);
+                else missed += weight * here;
+            }
+        }
+    }
+    if (!tiles) return f;
+    f.words = words / samples;
+    f.missed = missed / samples;
+    f.length = length / tiles;
+    return f;
 }
 
-bool rs_stage_supported(const DevGeom& g, tomo_dtype dt) {
-    if (!rs_stage_fits(g)) return false;
-    if (dt == TOMO_F32) return true;
-    // 16-bit volumes gain about a tenth of the projection for a second fill of 8 B a voxel: not
-    // below 128^3 (BF16, 64^3, 60 views: 71 us against 61; 128^3, 128 views: 477 against 492),
-    // nor with few samples per voxel
-    const double vox = (double)g.nx * g.ny * g.nz, samples = (double)g.np * g.nu * g.nv * std::max(g.nx, g.ny);
-    return vox >= 2097152.0 && samples >= 40.0 * vox;
+// Whether staging is the faster. A projection's time over that of the texture's gathers was
+// measured for 190 FP32 and 130 16-bit geometries (20^3 .. 256^3, 8 .. 300 views, pixels of
+// 0.12 .. 1.3 voxels at the centre, sources from 0.75 to 5 volume widths away, flat and deep
+// volumes) and fits: staged words per sample, the share of the samples whose window fits no stage
+// and that read global memory, and the wait for a block's first chunks over its rays' length,
+// which shows more where there are few blocks. E.g. FP32 160^3: 0.46 (0.25 voxels a pixel), 0.57
+// (1.0), 0.76 (1.3), 1.33 (1.3, source 0.75 widths away); 33 x 33 x 500: 2.6. 16-bit volumes,
+// which also pay a second fill: 0.89 (200^3, 60 views, 0.5 voxels), 0.98 (1.0), 1.11 (1.2);
+// 128^3 1.04 (64 views), 0.99 (128); below 128^3 1.02 to 1.4 from 0.5 voxels on; 300 x 300 x 30
+// (2400 blocks) 1.03.
+bool rs_stage_pays(const RsStageFit& f, const DevGeom& g, tomo_dtype dt) {
+    if (!f.fits) return false;
+    const double vox = (double)g.nx * g.ny * g.nz, rays = (double)g.np * g.nu * g.nv;
+    const double blocks = (double)g.np * rs_tiles_u(g) * rs_tiles_v(g);
+    if (dt == TOMO_F32) {
+        const double warp = g.rs_wlog == 3 ? 0.0 : g.rs_wlog == 4 ? 0.07 : 0.17;  // wider warps: more bank conflicts
+        return 0.357 + 0.095 * f.words + 6.4 * f.missed + (4.7 + 6.3 * std::min(1.0, 900 / blocks)) / f.length + warp < 0.905;
+    }
+    return vox >= 2097152.0 && blocks >= 3000 &&
+           0.663 + 0.074 * f.words + 5.5 * f.missed + 3.5 * vox / (rays * f.length) + 16.7 / f.length < 0.99;
 }
 
 // Copies of up to 64 MiB come from a pool of their device that keeps as much of what is freed, so

@@ -362,8 +362,12 @@ struct RsStage {
     int device = 0;      // current when they are made and destroyed
     bool pooled = false; // from the device's pool
 };
-bool rs_stage_fits(const DevGeom& g);                      // the tiles' windows fit the stages
-bool rs_stage_supported(const DevGeom& g, tomo_dtype dt);  // ... and staging is the faster
+struct RsStageFit {
+    bool fits = false;                       // the tiles' windows fit the stages
+    double words = 0, missed = 0, length = 1;  // staged words per sample, share of samples not staged, samples per ray
+};
+RsStageFit rs_stage_fit(const DevGeom& g, tomo_dtype dt);
+bool rs_stage_pays(const RsStageFit& f, const DevGeom& g, tomo_dtype dt);
 cudaError_t rs_stage_create(int nx, int ny, int nz, tomo_dtype dt, RsStage* t);
 void rs_stage_destroy(RsStage* t);
 void rs_stage_trim(int device);  // gives back what freed copies left in the device's pool
