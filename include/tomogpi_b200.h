@@ -206,13 +206,15 @@ tomo_status tomo_project_noalloc(const tomo_config_ct* cfg, int device, tomo_pro
 tomo_status tomo_count_samples(tomo_context* ctx, tomo_projector kind, unsigned long long* out, void* stream);
 
 /* Device error word of the context (bit 0: a Siddon traversal hit its step bound, bit 1:
-   a bounded wait gave up). Synchronous; clear != 0 resets it. */
+   a bounded wait gave up, i.e. the result of a staged projection or backprojection, on device
+   pointers, is undefined; the host-buffer forms report that as TOMO_ERR_TIMEOUT and clear the
+   bit). Synchronous; clear != 0 resets it. */
 tomo_status tomo_context_errors(tomo_context* ctx, unsigned* bits, int clear);
 /* For tests of the bounded waits only (no counterpart in the reference): with enable != 0,
-   the TMA-staged projections and backprojections of this context issue no copies, so every
-   wait of their consumers runs out after its one-second bound; the call completes with the
-   result undefined and bit 1 (a bounded wait gave up) set in the error word, and the
-   context stays usable. Never enabled otherwise. */
+   the TMA-staged projections and backprojections of this context and its solvers issue no
+   copies, so every wait of their consumers runs out after its one-second bound; the call
+   completes with the result undefined and bit 1 (a bounded wait gave up) set in the error
+   word, and the context stays usable. Never enabled otherwise. */
 tomo_status tomo_context_test_stall(tomo_context* ctx, int enable);
 /* For tests of what happens without device memory only: after `skip` more device allocations
    of the context and of its solvers, the next `count` are answered as out of memory, without

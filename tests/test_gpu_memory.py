@@ -236,3 +236,26 @@ def test_capture_with_a_sinogram_that_needs_rows(tomo):
         assert torch.equal(back, ref)
         torch.cuda.synchronize()
         del g
+
+
+@pytest.mark.parametrize("what", ["project", "backproject", "iterate"])
+def test_host_forms_report_a_wait_that_gave_up(tomo, what):
+    """A bounded wait that runs out (the test stall: no copies are issued) fails a call on host
+    buffers with TOMO_ERR_TIMEOUT; the next call is exact. One view of a tiny volume."""
+    from tomogpi_b200 import _lib as L
+
+    cfg = tomo.ConfigCT.cone_beam(16, 4)
+    vol = np.random.default_rng(3).random(cfg.volume_shape, dtype=np.float32)
+    with tomo.Context(cfg, views=(0, 1)) as ctx:
+        ctx.set_staging("fits")
+        s = np.random.default_rng(4).random(ctx.sinogram_shape, dtype=np.float32)
+        sv = tomo.Solver(ctx, _params(tomo))
+        call = {"project": lambda: ctx.project_host("RS", vol), "backproject": lambda: ctx.backproject_host("VI", s),
+                "iterate": lambda: sv.iterate_host(vol.copy(), s, first=1, count=1)}[what]
+        ref = call()
+        L.call("tomo_context_test_stall", ctx.handle, 1)
+        with pytest.raises(L.TomoError, match="TIMEOUT"):
+            call()
+        L.call("tomo_context_test_stall", ctx.handle, 0)
+        sv.set_state(-0.0347711, 1)
+        assert np.array_equal(call(), ref) and ctx.errors() == 0

@@ -660,6 +660,19 @@ tomo_status tomo_ramp_filter(tomo_context* ctx, const void* sinogram, tomo_dtype
                         "ramp_filter_kernel");
 }
 
+// The end of a call that returns host results: waits for its stream, and reports a bounded wait of
+// its kernels that gave up (the results are undefined then; the error bit is cleared).
+static tomo_status finish_host(tomo_context* ctx, cudaStream_t st) {
+    unsigned bits = 0;
+    TOMO_CUDA_TRY(cudaMemcpyAsync(&bits, ctx->d_err, sizeof(bits), cudaMemcpyDeviceToHost, st));
+    TOMO_CUDA_TRY(cudaStreamSynchronize(st));
+    if (!(bits & ERR_TIMEOUT)) return TOMO_OK;
+    bits &= ~ERR_TIMEOUT;
+    TOMO_CUDA_TRY(cudaMemcpy(ctx->d_err, &bits, sizeof(bits), cudaMemcpyHostToDevice));
+    set_error("a bounded wait of a staged kernel ran out; the result is undefined");
+    return TOMO_ERR_TIMEOUT;
+}
+
 tomo_status tomo_ramp_filter_host(tomo_context* ctx, const float* sinogram, float* out, int32_t oversampling,
                                   double cutoff) {
     TOMO_CHECK_ARG(ctx && sinogram && out, "tomo_ramp_filter_host: null argument");
@@ -688,8 +701,7 @@ tomo_status tomo_project_host(tomo_context* ctx, tomo_projector kind, const floa
     TOMO_CUDA_TRY(cudaMemcpyAsync(ctx->h_vol, volume, ctx->nvox() * sizeof(float), cudaMemcpyHostToDevice, st));
     if ((s = tomo_project(ctx, kind, ctx->h_vol, TOMO_F32, ctx->h_sino, TOMO_F32, st)) != TOMO_OK) return s;
     TOMO_CUDA_TRY(cudaMemcpyAsync(sinogram, ctx->h_sino, ctx->nsino() * sizeof(float), cudaMemcpyDeviceToHost, st));
-    TOMO_CUDA_TRY(cudaStreamSynchronize(st));
-    return TOMO_OK;
+    return finish_host(ctx, st);
 }
 
 tomo_status tomo_backproject_host(tomo_context* ctx, tomo_backprojector kind, const float* sinogram, float* volume) {
@@ -703,8 +715,7 @@ tomo_status tomo_backproject_host(tomo_context* ctx, tomo_backprojector kind, co
     TOMO_CUDA_TRY(cudaMemcpyAsync(ctx->h_sino, sinogram, ctx->nsino() * sizeof(float), cudaMemcpyHostToDevice, st));
     if ((s = tomo_backproject(ctx, kind, ctx->h_sino, TOMO_F32, ctx->h_vol, TOMO_F32, st)) != TOMO_OK) return s;
     TOMO_CUDA_TRY(cudaMemcpyAsync(volume, ctx->h_vol, ctx->nvox() * sizeof(float), cudaMemcpyDeviceToHost, st));
-    TOMO_CUDA_TRY(cudaStreamSynchronize(st));
-    return TOMO_OK;
+    return finish_host(ctx, st);
 }
 
 tomo_status tomo_count_samples(tomo_context* ctx, tomo_projector kind, unsigned long long* out, void* stream) {
@@ -956,7 +967,7 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
     };
     auto rs_project = [&](int epi, tomo_dtype odt, double* norm) -> cudaError_t {
         const int um = P.projector == TOMO_PROJ_RS ? 0 : 1;
-        if (sv->stage.rows) return launch_rs_stage(um, epi, g, sv->stage, sv->tex.tex, resid, odt, realv, rd, norm, ctx->d_err, st);
+        if (sv->stage.rows) return launch_rs_stage(um, epi, g, sv->stage, sv->tex.tex, resid, odt, realv, rd, norm, ctx->d_err, st, ctx->test_stall);
         return launch_rs_project(sv->rs_layout, um, epi, g, sv->vpad, sv->tex.tex, sd, resid, odt, realv, norm, st, rd);
     };
     for (int it = first; it < first + count; ++it) {
@@ -1019,7 +1030,7 @@ static tomo_status solver_run(tomo_solver* sv, float* volume, const void* real_s
                 if ((s = check_launch(sv->vtex.tex ? launch_vi_back_tex(um, g, sv->vtex.tex, TOMO_F32, sv->dJ, TOMO_F32, -2.0f,
                                                                         st, ctx->tuning.vi_zc)
                                       : sv->vi_tma ? launch_vi_back_tma(um, g, (const float*)sv->spad, vi_rows_pitch(g.nu), sv->dJ,
-                                                                        TOMO_F32, -2.0f, ctx->d_err, st)
+                                                                        TOMO_F32, -2.0f, ctx->d_err, st, ctx->test_stall)
                                                    : launch_vi_back(um, g, sv->spad, TOMO_F32, sv->dJ, TOMO_F32, -2.0f, st,
                                                                     ctx->tuning.vi_zc),
                                       "vi back")) != TOMO_OK)
@@ -1166,8 +1177,7 @@ tomo_status tomo_solver_iterate_host(tomo_solver* sv, float* volume, const void*
     }
     if (s != TOMO_OK) return s;
     TOMO_CUDA_TRY(cudaMemcpyAsync(volume, sv->d_vol, ctx->nvox() * sizeof(float), cudaMemcpyDeviceToHost, st));
-    TOMO_CUDA_TRY(cudaStreamSynchronize(st));
-    return TOMO_OK;
+    return finish_host(ctx, st);
 }
 
 tomo_status tomo_solver_set_timing(tomo_solver* sv, int enable) {
