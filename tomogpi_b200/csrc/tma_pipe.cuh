@@ -25,9 +25,13 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-// Waits for the phase of parity `parity` to complete; false once a second has passed (the
-// clock is read every 256 polls; a poll may itself suspend the thread for a short while).
-__device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity) {
+// Waits for the phase of parity `parity` to complete, as a whole warp; false once a second has
+// passed (the clock is read every 256 polls; a poll may itself suspend the thread for a short
+// while). One answer for the 32 lanes, which may see the phase or the second pass at different
+// polls: they vote at every poll, so all control flow and __syncwarp() after a wait that gave up
+// stay uniform over the warp. (A phase that one lane has seen stays visible to the others: the
+// next one needs this warp's arrival.)
+__device__ __forceinline__ bool mbar_wait_warp(unsigned long long* b, unsigned parity) {
     unsigned long long t0 = 0;
     for (unsigned i = 0;; ++i) {
         unsigned done;
@@ -38,18 +42,13 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity
             : "=r"(done)
             : "r"(smem_addr(b)), "r"(parity)
             : "memory");
-        if (done) return true;
+        if (__all_sync(0xffffffffu, done)) return true;
         if ((i & 255u) == 0) {
             const unsigned long long t = global_ns();
             if (i == 0) t0 = t;
-            else if (t - t0 > PIPE_WAIT_NS) return false;
+            else if (__any_sync(0xffffffffu, t - t0 > PIPE_WAIT_NS)) return false;
         }
     }
-}
-// The same for a whole warp: one answer for its 32 lanes, which may see the second pass at
-// different polls. All later control flow and __syncwarp() stay uniform over the warp.
-__device__ __forceinline__ bool mbar_wait_warp(unsigned long long* b, unsigned parity) {
-    return __all_sync(0xffffffffu, mbar_wait(b, parity));
 }
 __device__ __forceinline__ void tma_load_3d(float* dst, const CUtensorMap* map, int c0, int c1, int c2,
                                             unsigned long long* bar) {
