@@ -18,8 +18,8 @@
 //          sample is two (one) 128-bit loads from a single sector. 8x the volume's bytes.
 //   TEX    2D layered array in the storage type (raw 16-bit for BF16/FP16), slice z in
 //          layer z + 1 between two zero layers; two 4-texel tld4 gathers per sample. FP32
-//          volumes are staged in shared memory instead where the geometry allows it
-//          (rs_stage.cuh; this texture when it does not, or without memory for the copies).
+//          volumes are staged in shared memory instead where that is the faster
+//          (rs_stage.cuh; this texture elsewhere, and without memory for the copies).
 //   HYBRID TEX for the lower slice of a sample plus, for the upper slice, quads (the slice's
 //          four footprint texels in tld4 order, 16 B FP32 / 8 B 16-bit) in global memory, in a
 //          row-major and a column-major array: one gather and one 128-bit load per sample.

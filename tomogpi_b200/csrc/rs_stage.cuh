@@ -23,8 +23,7 @@
 // cp.async.bulk.tensor per plane (no multicast; this GPU's own buffer; texels off the volume
 // come back as the copy's zero fill, which is the reference's texture border). The window's
 // width W is one of a few values that put the four rows (z) of a warp's 8 u x 4 v rays on
-// different banks (256^3: {24, 40, 52, 68, 84} 7.25 ms, {24, 40, 56, 72, 88} 7.36,
-// {36, 44, 52, 68, 84} 7.75). The rays of a block stay within a
+// different banks (256^3: {24, 40, 56, 72, 88} takes 1.5% longer, {36, 44, 52, 68, 84} 7%). The rays of a block stay within a
 // chunk of each other, so a plane is staged once per block.
 //
 // A ray's samples are the repeated additions and the arithmetic of rs_device.cuh whatever
@@ -45,8 +44,8 @@ namespace tomo {
 
 constexpr int RSG_THREADS = 256 + 32;  // consumers (one ray each), producer warp
 constexpr int RSG_STAGES = 2;
-// Words of a stage: four blocks of two 27 KB stages per SM (256^3, 256 views, blocks x words:
-// 2 x 12288 8.25 ms, 3 x 8192 7.43, 4 x 6912 7.34, 5 x 5440 7.74, 6 x 4608 8.71: more blocks
+// Words of a stage: four blocks of two 27 KB stages per SM (256^3, 256 views, blocks x words
+// against 4 x 6912: 2 x 12288 12% longer, 3 x 8192 1%, 5 x 5440 5%, 6 x 4608 19%: more blocks
 // hide the waits at chunk ends, shorter chunks stage their two shared planes more often).
 constexpr int RSG_CAP = 6912, RSG_MIN_BLOCKS = 4;
 // Sixteenths of the blocks that gather from the packed texture instead (16-bit volumes): the
@@ -92,7 +91,6 @@ struct RsStageShared {
     int lo, hi;                  // plane floors of the block's samples
     float st[2], sz[2];          // range of the corner rays' slopes: t and z per plane
     int along;                   // the corner rays run along the march axis
-    int abort_flag;
 };
 constexpr int RSG_HEADER = 512;  // bytes before the stages
 static_assert(sizeof(RsStageShared) <= RSG_HEADER, "the stages start after the header");
@@ -105,7 +103,6 @@ __device__ __forceinline__ void rsg_init(RsStageShared* sh) {
             mbar_init(&sh->full[s], 1);
             mbar_init(&sh->empty[s], 8);  // one arrival per consumer warp
         }
-        sh->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
 }
@@ -232,11 +229,8 @@ __device__ __forceinline__ void rsg_produce(const DevGeom& g, const RsStageMaps&
         const int s = turn % RSG_STAGES;
         const unsigned k = turn / RSG_STAGES;
         if (k > 0 && !mbar_wait_warp(&sh->empty[s], (k - 1) & 1)) {
-            if (lane == 0) {
-                atomicOr(err, ERR_TIMEOUT);
-                sh->abort_flag = 1;
-            }
-            break;
+            if (lane == 0) atomicOr(err, ERR_TIMEOUT);
+            break;  // the consumers' waits run out as well
         }
         const int best = ok ? 31 - __clz(ok) : min(8, left) - 1;  // not staged: eight planes from global memory
         const int n = best + 1;
@@ -357,7 +351,6 @@ __device__ __forceinline__ void rs_stage_tile(const DevGeom& g, const RsStageMap
                     if (lane == 0) atomicOr(err, ERR_TIMEOUT);
                     break;
                 }
-                if (__any_sync(0xffffffffu, *(volatile int*)&sh->abort_flag)) break;
                 const RsChunk ch = sh->chunk[s];
                 // samples before the chunk's edge; one within 0.1 of it waits for the next chunk,
                 // whose planes start one earlier

@@ -351,7 +351,7 @@ void rs_tex_destroy(RsTexture* t);
 cudaError_t rs_tex_fill(const void* vol, tomo_dtype vdt, int nx, int ny, int nz, const RsTexture& t, cudaStream_t st,
                         const unsigned* amax = nullptr);
 // STAGE resources (rs_stage.cuh): the volume's two copies in 32-bit words (FP32, or pairs of
-// 16-bit slices) and their tensor maps. What TEX stands for wherever the geometry allows it;
+// 16-bit slices) and their tensor maps. What TEX stands for where that is the faster (rs_stage_pays);
 // 16-bit volumes have the packed texture beside them, which part of the blocks gather from.
 struct RsStageMaps;
 struct RsStage {
