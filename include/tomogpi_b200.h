@@ -119,10 +119,10 @@ tomo_status tomo_context_geometry(const tomo_context* ctx, float* scalars, float
    0 = zero-bordered padded copy (1x), 1 = 2x2x2 texel cells (8x the volume's bytes, one
    aligned 32 B / 16 B vector load per sample), 2 = 2D layered texture in the storage type
    (FP32, or the raw bits of BF16 / FP16), one layer per z slice, read with 4-texel gathers
-   (depths beyond the device's layer limit use 1) -- or, where a detector tile's windows of
-   the volume fit, staged in shared memory by TMA from two copies of it (8 B a voxel; FP32 in
-   place of the texture, 16-bit volumes from 128^3 on beside it), the same results --, 3 = the texture for the lower slice of
-   each sample plus, for the upper slice, the slice's four footprint texels stored together
+   (depths beyond the device's layer limit use 1) -- or, where that is the faster
+   (tomo_context_set_staging), staged in shared memory by TMA from two copies of the volume (8 B
+   a voxel; FP32 in place of the texture, 16-bit beside it), the same results --, 3 = the
+   texture for the lower slice of each sample plus, for the upper slice, the slice's four footprint texels stored together
    (FP32 only; 8x the volume's bytes besides the texture), 4 = faces across the axis the
    view's rays mostly run along, even faces in a layered texture and odd faces as stored
    2 x 2 footprints, each sample reusing the faces it shares with the previous sample of its
@@ -135,7 +135,8 @@ tomo_status tomo_context_geometry(const tomo_context* ctx, float* scalars, float
    copy where needed), else a zero-bordered padded copy (four scalar loads per voxel and view),
    1 = 2D layered texture, one layer per view, one 4-texel gather per voxel and view (view
    counts beyond the layer limit use 0), 2 = FP32 sinogram windows staged in shared memory
-   by TMA, one per (voxel tile, view), read by the bilinear samples. Set before creating solvers on the context. */
+   by TMA, one per (voxel tile, view), read by the bilinear samples. Set before creating
+   solvers on the context. */
 typedef struct {
     int32_t rs_layout;
     int32_t vi_zc;       /* VI: 16-slice chunks per thread (1, 2 or 4; 0 = default 1) */

@@ -406,7 +406,7 @@ tomo_status tomo_context_create_views(const tomo_config_ct* cfg, int device, int
     ctx->device = device;
     // Measured on B200 (512^3, 512 views). RS, FP32: staged 109 ms (what TEX runs), hybrid 133,
     // texture gathers 218, 2x2x2 cells 269, padded scalar loads 367; BF16: staged and gathered
-    // 97, gathered 110, cells 155. VI: staged, 16 slices per thread 43.4 ms; padded 72, with 32
+    // 97, gathered 110, cells 155. VI: staged, 16 slices per thread 43.6 ms; padded 72, with 32
     // slices 79; the texture form of the sinogram 111.
     ctx->tuning.rs_layout = RS_LAYOUT_TEX;
     ctx->tuning.vi_zc = 1;

@@ -368,11 +368,19 @@ __device__ __forceinline__ void rs_tile(const DevGeom& g, const Tv* __restrict__
             auto march = [&](auto sample) {
                 float2 AB = make_float2(r.A, r.B);
                 float C = r.C;
-                for (unsigned n = 0; n < r.n; ++n) {
+                auto step = [&](unsigned n) {
                     const RsSample s = rs_sample(AB, C);
                     acc = fadd(acc, fmul(dx, sample(s, n)));  // :292
                     AB = __fadd2_rn(AB, SXY);              // :295-297
                     C = fadd(C, r.sz);
+                };
+                if constexpr (LAYOUT == RS_LAYOUT_TEX && sizeof(Tv) == 4) {
+                    // three samples' gathers in flight: small jobs (48^3 .. 130^3) up to 12% faster
+                    // than with the compiler's two, none slower
+#pragma unroll 3
+                    for (unsigned n = 0; n < r.n; ++n) step(n);
+                } else {
+                    for (unsigned n = 0; n < r.n; ++n) step(n);
                 }
             };
             if (LAYOUT == RS_LAYOUT_MARCH) {

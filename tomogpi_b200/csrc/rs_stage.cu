@@ -152,6 +152,7 @@ RsStageFit rs_stage_fit(const DevGeom& g, tomo_dtype dt) {
     f.words = words / samples;
     f.missed = missed / samples;
     f.length = length / tiles;
+    f.hit = tiles / (g.nx == g.ny ? 27.0 : 54.0);
     return f;
 }
 
@@ -168,12 +169,12 @@ RsStageFit rs_stage_fit(const DevGeom& g, tomo_dtype dt) {
 bool rs_stage_pays(const RsStageFit& f, const DevGeom& g, tomo_dtype dt) {
     if (!f.fits) return false;
     const double vox = (double)g.nx * g.ny * g.nz, rays = (double)g.np * g.nu * g.nv;
-    const double blocks = (double)g.np * rs_tiles_u(g) * rs_tiles_v(g);
     if (dt == TOMO_F32) {
+        const double full = f.hit * rays / 256;  // blocks' worth of rays through the volume
         const double warp = g.rs_wlog == 3 ? 0.0 : g.rs_wlog == 4 ? 0.07 : 0.17;  // wider warps: more bank conflicts
-        return 0.357 + 0.095 * f.words + 6.4 * f.missed + (4.7 + 6.3 * std::min(1.0, 900 / blocks)) / f.length + warp < 0.905;
+        return 0.33 + 0.101 * f.words + 5.7 * f.missed + (6.2 + 2.4 * std::min(3.0, 900 / full)) / f.length + warp < 0.885;
     }
-    return vox >= 2097152.0 && blocks >= 3000 &&
+    return vox >= 2097152.0 && (double)g.np * rs_tiles_u(g) * rs_tiles_v(g) >= 3000 &&
            0.663 + 0.074 * f.words + 5.5 * f.missed + 3.5 * vox / (rays * f.length) + 16.7 / f.length < 0.99;
 }
 

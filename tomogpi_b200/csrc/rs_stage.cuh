@@ -8,7 +8,7 @@
 // sample's eight 32-bit reads take 14.7 clocks per warp with their bank conflicts (the 32
 // lanes' texels lie in a patch of about 40 words, so two lanes of some bank usually differ).
 // Neighbouring rays share texels: about 3 words are copied in per sample. FP32, 256^3, 256
-// views: TEX 13.7 ms, HYBRID 8.4, STAGE 7.16, with the shared-memory reads at 87% of their
+// views: TEX 13.7 ms, HYBRID 8.4, STAGE 7.18, with the shared-memory reads at 87% of their
 // rate; 512^3: TEX 218 ms, HYBRID 133, STAGE 109. 16-bit volumes read four words of slice pairs
 // per sample and are bound by issue (60 instructions per sample at 85%), no faster than the
 // texture alone; together they are (RSG_SHARE16).

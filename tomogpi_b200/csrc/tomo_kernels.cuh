@@ -365,6 +365,7 @@ struct RsStage {
 struct RsStageFit {
     bool fits = false;                       // the tiles' windows fit the stages
     double words = 0, missed = 0, length = 1;  // staged words per sample, share of samples not staged, samples per ray
+    double hit = 0;                            // share of the tiles whose central ray crosses the volume
 };
 RsStageFit rs_stage_fit(const DevGeom& g, tomo_dtype dt);
 bool rs_stage_pays(const RsStageFit& f, const DevGeom& g, tomo_dtype dt);

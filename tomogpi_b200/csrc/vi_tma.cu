@@ -17,11 +17,11 @@
 // memory; a view whose window exceeds the box reads that view's texels from global memory
 // instead. Same texels, same operations, bit-identical to vi_tile.
 //
-// Measured (B200): 512^3, 512 views 44.1 ms (51.6 before the window checks moved from every
+// Measured (B200): 512^3, 512 views 43.6 ms (51.6 before the window checks moved from every
 // thread to the producer, the texture's 0.5 offsets went and the reads took byte addresses;
-// the padded form 72.3); 256^3 2.81 ms (padded 4.85); filter and FDK backprojection together 3.77 ms
+// the padded form 72.3); 256^3 2.80 ms (padded 4.85); filter and FDK backprojection together 3.80 ms
 // (padded 9.99: the weights take one reciprocal square root now, in place of an IEEE division and
-// root per sample); 64^3, 60 views 35 us (padded, 64 blocks of 16 slices: 148).
+// root per sample); 64^3, 60 views 37 us (padded, 64 blocks of 16 slices: 148).
 //
 // Every wait is bounded (one second by the global timer): a wait that gives up sets
 // ERR_TIMEOUT in the context's error word and the block stops; the producer first waits
