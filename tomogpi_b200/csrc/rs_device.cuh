@@ -345,8 +345,9 @@ __device__ __forceinline__ bool rs_ray_inside(const DevGeom& g, const RsRay& r) 
 // One 2^rs_tlog u x 2^(8 - rs_tlog) v tile of view p (256 threads; each warp's rays span
 // 2^rs_wlog u x 2^(5 - rs_wlog) v): ray set-up,
 // trilinear march, epilogue. Shared by the single-job kernel and the batched persistent
-// kernel (batch.cu); must be called by all threads of the block (EPI_NORM syncs).
-template <int MODE, int LAYOUT, typename Tv, typename To, int EPI, typename Tr = To>
+// kernel (batch.cu); must be called by all threads of the block (EPI_NORM syncs). DEEP: room for
+// the registers of three FP32 samples at a time (the batch's kernels have 48 per thread).
+template <int MODE, int LAYOUT, typename Tv, typename To, int EPI, typename Tr = To, bool DEEP = false>
 __device__ __forceinline__ void rs_tile(const DevGeom& g, const Tv* __restrict__ vin, unsigned long long tex,
                                         const OutView<To>& out, const OutView<Tr>& real, double* __restrict__ norm,
                                         int p, int ut, int vt) {
@@ -374,7 +375,7 @@ __device__ __forceinline__ void rs_tile(const DevGeom& g, const Tv* __restrict__
                     AB = __fadd2_rn(AB, SXY);              // :295-297
                     C = fadd(C, r.sz);
                 };
-                if constexpr (LAYOUT == RS_LAYOUT_TEX && sizeof(Tv) == 4) {
+                if constexpr (DEEP && LAYOUT == RS_LAYOUT_TEX && sizeof(Tv) == 4) {
                     // three samples' gathers in flight: small jobs (48^3 .. 130^3) up to 12% faster
                     // than with the compiler's two, none slower
 #pragma unroll 3

@@ -112,7 +112,7 @@ rs_project_kernel(DevGeom g, const Tv* __restrict__ vin, unsigned long long tex,
         const int p = __ldg(g.view_order + (other ? g.view_cols + i : i));
         rs_tile<MODE, LAYOUT, Tv, To, EPI, Tr>(g, vin, tex, out, real, norm, p, blockIdx.y, blockIdx.z - (other ? tv : 0));
     } else {
-        rs_tile<MODE, LAYOUT, Tv, To, EPI, Tr>(g, vin, tex, out, real, norm, blockIdx.x, blockIdx.y, blockIdx.z);
+        rs_tile<MODE, LAYOUT, Tv, To, EPI, Tr, true>(g, vin, tex, out, real, norm, blockIdx.x, blockIdx.y, blockIdx.z);
     }
 }
 
