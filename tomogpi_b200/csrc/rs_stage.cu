@@ -157,11 +157,11 @@ RsStageFit rs_stage_fit(const DevGeom& g, tomo_dtype dt) {
 }
 
 // Whether staging is the faster. A projection's time over that of the texture's gathers was
-// measured for 190 FP32 and 130 16-bit geometries (20^3 .. 256^3, 8 .. 300 views, pixels of
+// measured for 600 FP32 and 170 16-bit geometries (16^3 .. 288^3, 8 .. 300 views, pixels of
 // 0.12 .. 1.3 voxels at the centre, sources from 0.75 to 5 volume widths away, flat and deep
 // volumes) and fits: staged words per sample, the share of the samples whose window fits no stage
 // and that read global memory, and the wait for a block's first chunks over its rays' length,
-// which shows more where there are few blocks. E.g. FP32 160^3: 0.46 (0.25 voxels a pixel), 0.57
+// which shows more where few rays cross the volume. None of them is staged at a loss. E.g. FP32 160^3: 0.46 (0.25 voxels a pixel), 0.57
 // (1.0), 0.76 (1.3), 1.33 (1.3, source 0.75 widths away); 33 x 33 x 500: 2.6. 16-bit volumes,
 // which also pay a second fill: 0.89 (200^3, 60 views, 0.5 voxels), 0.98 (1.0), 1.11 (1.2);
 // 128^3 1.04 (64 views), 0.99 (128); below 128^3 1.02 to 1.4 from 0.5 voxels on; 300 x 300 x 30
@@ -174,8 +174,10 @@ bool rs_stage_pays(const RsStageFit& f, const DevGeom& g, tomo_dtype dt) {
         const double warp = g.rs_wlog == 3 ? 0.0 : g.rs_wlog == 4 ? 0.07 : 0.17;  // wider warps: more bank conflicts
         return 0.33 + 0.101 * f.words + 5.7 * f.missed + (6.2 + 2.4 * std::min(3.0, 900 / full)) / f.length + warp < 0.885;
     }
-    return vox >= 2097152.0 && (double)g.np * rs_tiles_u(g) * rs_tiles_v(g) >= 3000 &&
-           0.663 + 0.074 * f.words + 5.5 * f.missed + 3.5 * vox / (rays * f.length) + 16.7 / f.length < 0.99;
+    const double blocks = (double)g.np * rs_tiles_u(g) * rs_tiles_v(g);  // 256 blocks / rays: partial tiles
+    return vox >= 2097152.0 && blocks >= 3000 &&
+           0.453 + 0.0523 * f.words + 5.5 * f.missed + 3.68 * vox / (rays * f.length) + 11.2 / f.length +
+                   0.281 * 256 * blocks / rays < 0.985;
 }
 
 // Copies of up to 64 MiB come from a pool of their device that keeps as much of what is freed, so
