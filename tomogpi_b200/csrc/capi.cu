@@ -212,9 +212,9 @@ tomo_status solver_texture(tomo_solver* sv) {
     return TOMO_OK;
 }
 
-// A buffer of the solver's: the context's and its own staged copies give way to it. The texture that takes their
-// place is made before the buffer; without room for it the solver has neither until solver_run
-// makes it, and the buffer is not handed out.
+// A buffer of the solver's: the context's and its own staged copies give way to it. The texture
+// that takes their place is made before the buffer; without room for it the solver has neither
+// until solver_run makes it, and the buffer is not handed out.
 tomo_status ensure(tomo_solver* sv, void** p, size_t bytes, bool zero) {
     tomo_status s = ensure(sv->ctx, p, bytes, zero);
     if (s != TOMO_ERR_NO_MEMORY || !sv->stage.rows || sv->stage_held) return s;
